@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "cumc_round.cuh"
+
 namespace cumc {
 
 constexpr int NG = 3;  // ghost layers (solver/definition.f90:54)
@@ -74,9 +76,28 @@ enum { IRHO = 0, IVX = 1, IVY = 2, IVZ = 3, ITAU = 4, IBX = 5, IBY = 6, IBZ = 7 
 // (solver/reconstruct.f90:254-280). The reference evaluates this three times
 // per call (dmm1, dmc, dmp1); the three forms are the same expression of the
 // cell's own (vm, vc, vp) and weights, so it is computed once per cell.
+//
+// The sweeps are bound by the FP64 pipe, so the double forms here and below
+// move what they can to the integer pipe without changing a value: signs and
+// minima of products and magnitudes are read from the bit patterns (a double
+// orders like its bits among the non-negative ones), a product with 2 merges
+// with the following sum (it is exact, so the fused sum rounds the same), and
+// min(2a, 2b) = 2 min(a, b).
+__device__ __forceinline__ bool is_pos(double x) { return __double_as_longlong(x) > 0; }
+__device__ __forceinline__ bool is_neg(double x) {
+    return (unsigned long long)__double_as_longlong(x) > 0x8000000000000000ull;
+}
+__device__ __forceinline__ double min_mag(double a, double b) {  // both non-negative
+    return __longlong_as_double(min(__double_as_longlong(a), __double_as_longlong(b)));
+}
 template <typename R>
 __device__ __forceinline__ R ppm_slope(R vm, R vc, R vp, R b0, R b1) {
     const R delta = b0 * (vp - vc) + b1 * (vc - vm);
+    if constexpr (sizeof(R) == 8) {
+        const double up = vp - vc, dn = vc - vm;
+        const double s = copysign(min_mag(fabs(delta), 2.0 * min_mag(fabs(dn), fabs(up))), delta);
+        return is_pos(up * dn) ? s : 0.0;
+    }
     if ((vp - vc) * (vc - vm) > R(0))
         return fmin(fmin(fabs(delta), R(2) * fabs(vc - vm)), R(2) * fabs(vc - vp)) * copysign(R(1), delta);
     return R(0);
@@ -93,6 +114,16 @@ __device__ __forceinline__ R ppm_face(R vc, R vp, R dmc, R dmp, R a0, R a1, R a2
 // The second test reads the already-modified left value, as the reference does.
 template <typename R>
 __device__ __forceinline__ void ppm_fix(R vc, R vl, R vr, R& vm_out, R& vp_out) {
+    if constexpr (sizeof(R) == 8) {
+        const double c3 = 3.0 * vc;
+        const bool flat = !is_pos((vr - vc) * (vc - vl));
+        const double m = is_neg((vr - vl) * __fma_rn(2.0, vr, vl - c3)) ? __fma_rn(-2.0, vr, c3) : vl;
+        const double q = __fma_rn(-2.0, vl, c3);
+        const double p = is_neg((vr - m) * (q - vr)) ? q : vr;
+        vm_out = flat ? vc : m;
+        vp_out = flat ? vc : p;
+        return;
+    }
     vm_out = vl;
     vp_out = vr;
     if ((vr - vc) * (vc - vl) <= R(0)) {
@@ -129,6 +160,16 @@ __device__ __forceinline__ R signalspeed(R cs, R bn, R bt1, R bt2, R rho) {
     return sqrt(R(0.5) * ((a2 + b2) + sqrt(fmax(((a4 + b4) + (R(2) * b2) * a2) - (R(4) * a2) * b2n, R(0)))));
 }
 
+// 1/x, sqrt(x) and sqrt(max(x, 0)) of the reciprocal form: in FP64 by
+// Newton-Raphson without a branch (within a unit in the last place), in FP32
+// the IEEE operations
+__device__ __forceinline__ double recip_r(double x) { return recip_near(x, recip_seed(x)); }
+__device__ __forceinline__ float recip_r(float x) { return 1.0f / x; }
+__device__ __forceinline__ double sqrt_r(double x) { return root_pos(x); }
+__device__ __forceinline__ float sqrt_r(float x) { return sqrtf(x); }
+__device__ __forceinline__ double sqrt_max0(double x) { return root_pos(x); }
+__device__ __forceinline__ float sqrt_max0(float x) { return sqrtf(fmaxf(x, 0.0f)); }
+
 // compute_signalspeed with the quotients by rho formed as products with
 // irho = 1/rho (the CUMC_FP64_FAST form: not bit-compatible with the reference)
 template <typename R>
@@ -140,7 +181,7 @@ __device__ __forceinline__ R signalspeed_recip(R cs, R bn, R bt1, R bt2, R irho)
     const R b2t2 = (bt2 * bt2) * irho;
     const R b2 = (b2n + b2t1) + b2t2;
     const R b4 = b2 * b2;
-    return sqrt(R(0.5) * ((a2 + b2) + sqrt(fmax(((a4 + b4) + (R(2) * b2) * a2) - (R(4) * a2) * b2n, R(0)))));
+    return sqrt_r(R(0.5) * ((a2 + b2) + sqrt_max0(((a4 + b4) + (R(2) * b2) * a2) - (R(4) * a2) * b2n)));
 }
 
 // compute_roe (solver/definition.f90:387-392)
@@ -213,18 +254,18 @@ __device__ __forceinline__ void hll_flux7(const R wl[8], const R wr[8], R ggas, 
     constexpr int ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
     using Side = FaceSide<DIR, R>;
     R sL, sR;
-    Side L = RECIP ? Side(wl, wl[ITAU] * (R(1) / wl[IRHO]) * (R(1) / (ggas - R(1))), typename Side::GivenEps{})
+    Side L = RECIP ? Side(wl, wl[ITAU] * recip_r(wl[IRHO]) * recip_r(ggas - R(1)), typename Side::GivenEps{})
                    : Side(wl, ggas);
-    Side Rs = RECIP ? Side(wr, wr[ITAU] * (R(1) / wr[IRHO]) * (R(1) / (ggas - R(1))), typename Side::GivenEps{})
+    Side Rs = RECIP ? Side(wr, wr[ITAU] * recip_r(wr[IRHO]) * recip_r(ggas - R(1)), typename Side::GivenEps{})
                     : Side(wr, ggas);
     if (RECIP) {
-        const R irL = R(1) / wl[IRHO], irR = R(1) / wr[IRHO];
-        const R csL = sqrt((ggas * wl[ITAU]) * irL);
-        const R csR = sqrt((ggas * wr[ITAU]) * irR);
+        const R irL = recip_r(wl[IRHO]), irR = recip_r(wr[IRHO]);
+        const R csL = sqrt_r((ggas * wl[ITAU]) * irL);
+        const R csR = sqrt_r((ggas * wr[ITAU]) * irR);
         const R cfsL = signalspeed_recip(csL, wl[ibn], wl[ibt1], wl[ibt2], irL);
         const R cfsR = signalspeed_recip(csR, wr[ibn], wr[ibt1], wr[ibt2], irR);
-        const R sqL = sqrt(wl[IRHO]), sqR = sqrt(wr[IRHO]);
-        const R isq = R(1) / (sqL + sqR);
+        const R sqL = sqrt_r(wl[IRHO]), sqR = sqrt_r(wr[IRHO]);
+        const R isq = recip_r(sqL + sqR);
         const R ubar = (sqL * wl[ivn] + sqR * wr[ivn]) * isq;
         const R cbar = (sqL * cfsL + sqR * cfsR) * isq;
         sL = fmin(wl[ivn] - cfsL, ubar - cbar);
@@ -249,7 +290,7 @@ __device__ __forceinline__ void hll_flux7(const R wl[8], const R wr[8], R ggas, 
         for (int c = 0; c < 7; ++c) out[c] = L.f(comp[c]);
     } else if (sL <= R(0) && sR >= R(0)) {
         if (RECIP) {
-            const R ids = R(1) / (sR - sL);
+            const R ids = recip_r(sR - sL);
 #pragma unroll
             for (int c = 0; c < 7; ++c) {
                 const R yl = L.f(comp[c]), yr = Rs.f(comp[c]), xl = L.u(comp[c]), xr = Rs.u(comp[c]);
@@ -264,6 +305,90 @@ __device__ __forceinline__ void hll_flux7(const R wl[8], const R wr[8], R ggas, 
 #pragma unroll
         for (int c = 0; c < 7; ++c) out[c] = Rs.f(comp[c]);
     }
+}
+
+// hll_flux7 with the plain operators, out of line: the faces whose operands
+// leave the ranges of hll_flux7_rounded
+template <int DIR>
+__device__ __noinline__ void hll_flux7_ieee(const double* w, double ggas, double* out) {
+    double wl[8], wr[8], fx[7];
+    for (int q = 0; q < 8; ++q) {
+        wl[q] = w[q];
+        wr[q] = w[8 + q];
+    }
+    hll_flux7<DIR, double>(wl, wr, ggas, fx);
+    for (int q = 0; q < 7; ++q) out[q] = fx[q];
+}
+
+// one side's fast speed and internal energy for hll_flux7_rounded; the values
+// of EOS_SOUNDSPEED, compute_signalspeed and EOS_EPSILON
+struct SideSpeed {
+    double cf, sq, e;
+};
+__device__ __forceinline__ SideSpeed side_speed(double rho, double p, double bn2, double bt1, double bt2, double ggas,
+                                                double gm1, const Recip& rg) {
+    const Recip r = recip_of(rho);
+    const double cs = root_of(quot(ggas * p, rho, r));
+    const double a2 = cs * cs;
+    const double b2n = quot(bn2, rho, r);
+    const double b2 = (b2n + quot(bt1 * bt1, rho, r)) + quot(bt2 * bt2, rho, r);
+    // ((a4 + b4) + (2 b2) a2) - (4 a2) b2n with the exact factors 2 and 4 merged
+    const double x = __fma_rn(2.0, b2 * a2, a2 * a2 + b2 * b2);
+    const double s = root_pos(__fma_rn(-4.0, a2 * b2n, x));
+    return {root_of(0.5 * ((a2 + b2) + s)), root_of(rho), quot(quot(p, rho, r), gm1, rg)};
+}
+
+// hll_flux7 in FP64, bit for bit, with the quotients and roots of
+// cumc_round.cuh. The sweeps are bound by the FP64 pipe and by its latency: the
+// 21 quotients and 8 roots of the plain form carried a range branch each, which
+// kept them from overlapping (1,414 instructions a face and warp in the y
+// walker, 0.53 issued a cycle at 160^3). y and z walkers 1.17 -> 0.88 ms and the
+// x sweep 1.25 -> 1.08 ms at 256^3 with the integer-pipe limiter above; the
+// torus' y walker 0.193 -> 0.108 ms. Returns false where an operand leaves their ranges and the face
+// needs the plain operators: a density or pressure outside [2^-200, 2^200), or
+// a nonzero HLL numerator below 2^-900. (Squared fields below 2^-900 need no
+// test: they vanish in the sums with a2 >= 2^-402.)
+template <int DIR>
+__device__ __forceinline__ bool hll_flux7_rounded(const double (&wl)[8], const double (&wr)[8], double ggas,
+                                                  double (&out)[7]) {
+    constexpr int ivn = IVX + DIR, ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
+    constexpr int bt_a = DIR == 0 ? IBY : IBX, bt_b = DIR == 2 ? IBY : IBZ;
+    constexpr int comp[7] = {IRHO, IVX, IVY, IVZ, ITAU, bt_a, bt_b};
+    const unsigned far =
+        range_max(wl[IRHO], range_max(wr[IRHO], range_max(wl[ITAU], range_max(wr[ITAU], 0u))));
+    if (far >= RANGE_SPAN) return false;
+    using Side = FaceSide<DIR, double>;
+    const double gm1 = ggas - 1.0, bn2 = wl[ibn] * wl[ibn];
+    const Recip rg = recip_of(gm1);
+    const SideSpeed l = side_speed(wl[IRHO], wl[ITAU], bn2, wl[ibt1], wl[ibt2], ggas, gm1, rg);
+    const SideSpeed r = side_speed(wr[IRHO], wr[ITAU], bn2, wr[ibt1], wr[ibt2], ggas, gm1, rg);
+    const double sq = l.sq + r.sq;
+    const Recip rs = recip_of(sq);
+    const double ubar = quot(l.sq * wl[ivn] + r.sq * wr[ivn], sq, rs);
+    const double cbar = quot(l.sq * l.cf + r.sq * r.cf, sq, rs);
+    const double sL = fmin(wl[ivn] - l.cf, ubar - cbar);
+    const double sR = fmax(wr[ivn] + r.cf, ubar + cbar);
+    const Side L(wl, l.e, typename Side::GivenEps{}), Rs(wr, r.e, typename Side::GivenEps{});
+    if (sL >= 0.0) {
+#pragma unroll
+        for (int c = 0; c < 7; ++c) out[c] = L.f(comp[c]);
+    } else if (sR >= 0.0) {
+        const double ds = sR - sL, lr = sL * sR;
+        const Recip rd = recip_of(ds);
+        unsigned tiny = ~0u;
+#pragma unroll
+        for (int c = 0; c < 7; ++c) {
+            const int q = comp[c];
+            const double a = (sR * L.f(q) - sL * Rs.f(q)) + lr * (Rs.u(q) - L.u(q));
+            tiny = tiny_min(a, tiny);
+            out[c] = quot_signed(a, ds, rd);
+        }
+        return tiny >= TINY;
+    } else {
+#pragma unroll
+        for (int c = 0; c < 7; ++c) out[c] = Rs.f(comp[c]);
+    }
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -485,8 +610,18 @@ __device__ __forceinline__ void sweep_hll(const R (&wl)[8], const R (&wr)[8], R 
     if constexpr (sizeof(R) == 4) {
         if constexpr (RECIP) hll_flux7<DIR, R, true>(wl, wr, ggas, fx);
         else hll_flux7_mixed<DIR>(wl, wr, ggas, fx);
-    } else {
-        hll_flux7<DIR, R, RECIP>(wl, wr, ggas, fx);
+    } else if constexpr (RECIP) {
+        hll_flux7<DIR, R, true>(wl, wr, ggas, fx);
+    } else if (!hll_flux7_rounded<DIR>(wl, wr, ggas, fx)) {
+        double w[16], f[7];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            w[q] = wl[q];
+            w[8 + q] = wr[q];
+        }
+        hll_flux7_ieee<DIR>(w, ggas, f);
+#pragma unroll
+        for (int q = 0; q < 7; ++q) fx[q] = f[q];
     }
 }
 
