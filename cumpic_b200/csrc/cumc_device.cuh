@@ -344,10 +344,10 @@ __device__ __forceinline__ SideSpeed side_speed(double rho, double p, double bn2
 // kept them from overlapping (1,414 instructions a face and warp in the y
 // walker, 0.53 issued a cycle at 160^3). y and z walkers 1.17 -> 0.88 ms and the
 // x sweep 1.25 -> 1.08 ms at 256^3 with the integer-pipe limiter above; the
-// torus' y walker 0.193 -> 0.108 ms. Returns false where an operand leaves their ranges and the face
-// needs the plain operators: a density or pressure outside [2^-200, 2^200), or
-// a nonzero HLL numerator below 2^-900. (Squared fields below 2^-900 need no
-// test: they vanish in the sums with a2 >= 2^-402.)
+// torus' y walker 0.193 -> 0.108 ms. Returns false where a density or pressure
+// lies outside [2^-200, 2^200) and the face needs the plain operators
+// throughout. (Squared fields below 2^-900 need no test: they vanish in the
+// sums with a2 >= 2^-402.)
 template <int DIR>
 __device__ __forceinline__ bool hll_flux7_rounded(const double (&wl)[8], const double (&wr)[8], double ggas,
                                                   double (&out)[7]) {
@@ -373,17 +373,14 @@ __device__ __forceinline__ bool hll_flux7_rounded(const double (&wl)[8], const d
 #pragma unroll
         for (int c = 0; c < 7; ++c) out[c] = L.f(comp[c]);
     } else if (sR >= 0.0) {
-        const double ds = sR - sL, lr = sL * sR;
-        const Recip rd = recip_of(ds);
-        unsigned tiny = ~0u;
+        const double lr = sL * sR;
+        double a[7];
 #pragma unroll
         for (int c = 0; c < 7; ++c) {
             const int q = comp[c];
-            const double a = (sR * L.f(q) - sL * Rs.f(q)) + lr * (Rs.u(q) - L.u(q));
-            tiny = tiny_min(a, tiny);
-            out[c] = quot_signed(a, ds, rd);
+            a[c] = (sR * L.f(q) - sL * Rs.f(q)) + lr * (Rs.u(q) - L.u(q));
         }
-        return tiny >= TINY;
+        quot_group(a, sR - sL, out);
     } else {
 #pragma unroll
         for (int c = 0; c < 7; ++c) out[c] = Rs.f(comp[c]);

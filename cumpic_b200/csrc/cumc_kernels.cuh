@@ -413,7 +413,7 @@ struct CellConv {
     double eps, p;    // p on the interior only
     bool bad;         // non-finite density, velocity or pressure (interior)
 };
-template <int MODEL, bool FROM_CONS>
+template <int MODEL, bool FROM_CONS, bool ROUNDED = false>
 __device__ __forceinline__ CellConv utop_of(const double* uh, bool interior, double bx, double by, double bz,
                                             double ggas, double rho_floor, double eps_floor) {
     CellConv o;
@@ -421,11 +421,21 @@ __device__ __forceinline__ CellConv utop_of(const double* uh, bool interior, dou
     double rho, vx, vy, vz, e;
     if (FROM_CONS) {
         rho = uh[IRHO];
-        vx = uh[IVX] / rho;
-        vy = uh[IVY] / rho;
-        vz = uh[IVZ] / rho;
-        const double vsquare = (vx * vx + vy * vy) + vz * vz;
-        e = (uh[ITAU] - 0.5 * bsquare) / rho - 0.5 * vsquare;
+        if constexpr (ROUNDED) {
+            const double a[4] = {uh[IVX], uh[IVY], uh[IVZ], uh[ITAU] - 0.5 * bsquare};
+            double q[4];
+            quot_group(a, rho, q);
+            vx = q[0];
+            vy = q[1];
+            vz = q[2];
+            e = q[3] - 0.5 * ((vx * vx + vy * vy) + vz * vz);
+        } else {
+            vx = uh[IVX] / rho;
+            vy = uh[IVY] / rho;
+            vz = uh[IVZ] / rho;
+            const double vsquare = (vx * vx + vy * vy) + vz * vz;
+            e = (uh[ITAU] - 0.5 * bsquare) / rho - 0.5 * vsquare;
+        }
     } else {
         rho = uh[0];
         vx = uh[1];
@@ -566,9 +576,88 @@ __device__ __forceinline__ void st2(double* p, int i, double x, double y) {
     *reinterpret_cast<double2*>(p + i) = make_double2(x, y);
 }
 
+// cell_dt with the quotients and roots of cumc_round.cuh: the same value
+// bit for bit, by the plain operators outside their ranges
+template <int COORD>
+__device__ __forceinline__ double cell_dt_rounded(const Tabs& T, int j, int k, int l, double rho, double p, double vx,
+                                                  double vy, double vz, double bcx, double bcy, double bcz,
+                                                  double ggas, double cfl) {
+    if (range_max(rho, range_max(p, 0u)) >= RANGE_SPAN)
+        return cell_dt<COORD>(T, j, k, l, rho, p, vx, vy, vz, bcx, bcy, bcz, ggas, cfl);
+    double dyl = T.ax[1].d[k], dzl = T.ax[2].d[l];
+    if (COORD != 1) cfl_lengths(COORD, T.ax[0].c[j], COORD == 3 ? T.sinc[k] : 0.0, dyl, dzl);
+    const Recip r = recip_of(rho);
+    const double cs = root_of(quot(ggas * p, rho, r));
+    const double a2 = cs * cs;
+    const double b2x = quot(bcx * bcx, rho, r), b2y = quot(bcy * bcy, rho, r), b2z = quot(bcz * bcz, rho, r);
+    const double b2 = (b2x + b2y) + b2z;
+    const double base = __fma_rn(2.0, a2 * b2, a2 * a2) + b2 * b2;
+    auto fast = [&](double b2d) {  // no MAX(., 0) under the inner root, as in cfl_cell_dt
+        const double x = __fma_rn(-4.0, a2 * b2d, base);
+        return root_of(0.5 * ((a2 + b2) + (x == 0.0 ? 0.0 : root_of(x))));
+    };
+    const double lambda = fmax(fmax(fabs(vx) + fast(b2x), fabs(vy) + fast(b2y)), fabs(vz) + fast(b2z));
+    const double num = fmin(fmin(T.ax[0].d[j], dyl), dzl) * cfl;
+    if (range_max(num, range_max(lambda, 0u)) >= RANGE_SPAN) return num / lambda;
+    return quot(num, lambda, recip_of(lambda));
+}
+
+// one direction's flux difference of the 5 hydro values of a pair's cells,
+// from the fluxes at the pair (c), below it (m: the same cells' lower faces
+// along y and z; along x the pair at i - 2, whose second value is cell 0's
+// lower face) and the GEOM_FLUX factors; cells outside the interior get a
+// zero numerator. SAME: both cells have one divisor.
+template <int COORD, int DIR>
+__device__ __forceinline__ void pair_flux_diff(const Tabs& T, const FaceFlux& f, int j, int k, int l, int i, int below,
+                                               bool in0, bool in1, double (&L0)[5], double (&L1)[5]) {
+    constexpr bool SAME = COORD == 1 ? DIR != 0 : COORD == 2 && DIR == 2;
+    double gp0, gc0, gm0, gp1, gc1, gm1;
+    geom_flux<COORD, DIR>(T, j, k, l, gp0, gc0, gm0);
+    geom_flux<COORD, DIR>(T, j + 1, k, l, gp1, gc1, gm1);
+    double a0[5], a1[5];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        const double2 c = ld2(f.f[q], i), m = ld2(f.f[q], below);
+        a0[q] = in0 ? c.x * gp0 - (DIR == 0 ? m.y : m.x) * gm0 : 0.0;
+        a1[q] = in1 ? c.y * gp1 - (DIR == 0 ? c.x : m.y) * gm1 : 0.0;
+    }
+    if constexpr (SAME) {
+        double a[10], r[10];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            a[q] = a0[q];
+            a[5 + q] = a1[q];
+        }
+        quot_group(a, gc0, r);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            L0[q] = L0[q] - r[q];
+            L1[q] = L1[q] - r[5 + q];
+        }
+    } else {
+        double r0[5], r1[5];
+        quot_group(a0, gc0, r0);
+        quot_group(a1, gc1, r1);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            L0[q] = L0[q] - r0[q];
+            L1[q] = L1[q] - r1[q];
+        }
+    }
+}
+
+// The quotients go through quot_group: 38 divisions with a branch each kept the
+// loads of one direction behind the quotients of the one before. Measured
+// (plain -> grouped): 1.23 -> 1.09-1.13 ms at 256^3, where its 5.7 GB then run
+// at 5.2 TB/s, 0.190 -> 0.155 ms on the 192x128x64 torus, 0.024 -> 0.015 ms on a
+// 512x4x4 tube. 4 blocks of 256 (64 registers); 3 take 1.12 and 2 take 1.32 ms.
+#ifndef CUMC_COMB_MINB
+#define CUMC_COMB_MINB 4
+#endif
 template <int COORD, int MODEL, int STAGE>
-__global__ void __launch_bounds__(256, 4) k_combine_utop2(Box b, Tabs T, Prim pr, FaceFlux fx, FaceFlux fy,
-                                                       FaceFlux fz, CombineArgs a, UtopArgs o) {
+__global__ void __launch_bounds__(256, CUMC_COMB_MINB) k_combine_utop2(Box b, Tabs T, Prim pr, FaceFlux fx,
+                                                                        FaceFlux fy, FaceFlux fz, CombineArgs a,
+                                                                        UtopArgs o) {
     if (b.skip && *b.skip) return;
     const int np = (b.nx + 2) >> 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -587,31 +676,9 @@ __global__ void __launch_bounds__(256, 4) k_combine_utop2(Box b, Tabs T, Prim pr
 #pragma unroll
         for (int q = 0; q < 5; ++q) L0[q] = L1[q] = 0.0;
         if (kl) {
-            double gp0, gc0, gm0, gp1, gc1, gm1;
-            geom_flux<COORD, 0>(T, j, k, l, gp0, gc0, gm0);
-            geom_flux<COORD, 0>(T, j + 1, k, l, gp1, gc1, gm1);
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                const double2 c = ld2(fx.f[q], i), m = ld2(fx.f[q], i - 2);
-                L0[q] = flux_diff(L0[q], c.x, m.y, gp0, gm0, gc0);
-                L1[q] = flux_diff(L1[q], c.y, c.x, gp1, gm1, gc1);
-            }
-            geom_flux<COORD, 1>(T, j, k, l, gp0, gc0, gm0);
-            geom_flux<COORD, 1>(T, j + 1, k, l, gp1, gc1, gm1);
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                const double2 c = ld2(fy.f[q], i), m = ld2(fy.f[q], i - sk);
-                L0[q] = flux_diff(L0[q], c.x, m.x, gp0, gm0, gc0);
-                L1[q] = flux_diff(L1[q], c.y, m.y, gp1, gm1, gc1);
-            }
-            geom_flux<COORD, 2>(T, j, k, l, gp0, gc0, gm0);
-            geom_flux<COORD, 2>(T, j + 1, k, l, gp1, gc1, gm1);
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                const double2 c = ld2(fz.f[q], i), m = ld2(fz.f[q], i - sl);
-                L0[q] = flux_diff(L0[q], c.x, m.x, gp0, gm0, gc0);
-                L1[q] = flux_diff(L1[q], c.y, m.y, gp1, gm1, gc1);
-            }
+            pair_flux_diff<COORD, 0>(T, fx, j, k, l, i, i - 2, in0, in1, L0, L1);
+            pair_flux_diff<COORD, 1>(T, fy, j, k, l, i, i - sk, in0, in1, L0, L1);
+            pair_flux_diff<COORD, 2>(T, fz, j, k, l, i, i - sl, in0, in1, L0, L1);
             double sc[5];
             if (in0) {
                 cell_sources<COORD, MODEL>(T, pr, a.geom_repeat, a.rho_floor, a.r_sh, j, k, l, i, sc);
@@ -675,8 +742,8 @@ __global__ void __launch_bounds__(256, 4) k_combine_utop2(Box b, Tabs T, Prim pr
                 o.bc[2][i + 1] = bz1;
             }
         }
-        const CellConv c0 = utop_of<MODEL, true>(uh0, in0, bx0, by0, bz0, o.ggas, o.rho_floor, o.eps_floor);
-        const CellConv c1 = utop_of<MODEL, true>(uh1, in1, bx1, by1, bz1, o.ggas, o.rho_floor, o.eps_floor);
+        const CellConv c0 = utop_of<MODEL, true, true>(uh0, in0, bx0, by0, bz0, o.ggas, o.rho_floor, o.eps_floor);
+        const CellConv c1 = utop_of<MODEL, true, true>(uh1, in1, bx1, by1, bz1, o.ggas, o.rho_floor, o.eps_floor);
         if (two) {
 #pragma unroll
             for (int q = 0; q < 5; ++q) st2(o.u[q], i, c0.u[q], c1.u[q]);
@@ -696,11 +763,11 @@ __global__ void __launch_bounds__(256, 4) k_combine_utop2(Box b, Tabs T, Prim pr
         if ((in0 && c0.bad) || (in1 && c1.bad)) atomicOr(o.flag, 1u);
         if (fuse_dt) {
             if (in0)
-                dt_cell = cell_dt<COORD>(T, j, k, l, c0.w[0], c0.p, c0.w[1], c0.w[2], c0.w[3], bx0, by0, bz0, o.ggas,
-                                         o.cfl);
+                dt_cell = cell_dt_rounded<COORD>(T, j, k, l, c0.w[0], c0.p, c0.w[1], c0.w[2], c0.w[3], bx0, by0, bz0,
+                                                 o.ggas, o.cfl);
             if (in1)
-                dt_cell = fmin(dt_cell, cell_dt<COORD>(T, j + 1, k, l, c1.w[0], c1.p, c1.w[1], c1.w[2], c1.w[3], bx1,
-                                                       by1, bz1, o.ggas, o.cfl));
+                dt_cell = fmin(dt_cell, cell_dt_rounded<COORD>(T, j + 1, k, l, c1.w[0], c1.p, c1.w[1], c1.w[2], c1.w[3],
+                                                               bx1, by1, bz1, o.ggas, o.cfl));
         }
     }
     if (fuse_dt) block_min_dt(dt_cell, o.dtmin);

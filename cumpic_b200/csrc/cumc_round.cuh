@@ -127,6 +127,28 @@ __device__ __forceinline__ unsigned tiny_min(double x, unsigned m) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     return __viaddmin_u32(hi + hi + min(lo, 1u), ~0u, m);
 }
+
+// a/b out of line, for the rare groups below
+static __device__ __noinline__ double plain_quot(double a, double b) { return a / b; }
+
+// q[n] = a[n]/b for N numerators, the shared reciprocal
+// where b and the numerators are in range, else the plain operator
+// (a front that fades into a zero field carries numerators down through the
+// denormals, so the test stands here and not around a whole face or cell)
+template <int N>
+__device__ __forceinline__ void quot_group(const double (&a)[N], double b, double (&q)[N]) {
+    unsigned tiny = ~0u;
+#pragma unroll
+    for (int n = 0; n < N; ++n) tiny = tiny_min(a[n], tiny);
+    if (range_max(b, 0u) < RANGE_SPAN && tiny >= TINY) {
+        const Recip r = recip_of(b);
+#pragma unroll
+        for (int n = 0; n < N; ++n) q[n] = quot_signed(a[n], b, r);
+    } else {
+#pragma unroll
+        for (int n = 0; n < N; ++n) q[n] = plain_quot(a[n], b);
+    }
+}
 #endif
 
 }  // namespace cumc
