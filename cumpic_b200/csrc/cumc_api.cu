@@ -238,6 +238,21 @@ void launch_grid(cumc_ctx* c, int cls, dim3 grid, int block, size_t smem, K kern
     }
 }
 
+// the default x sweep of the planes l_lo .. l_lo + l_cnt - 1; pairs move as
+// vectors with an even row stride
+void sweep_xpair(cumc_ctx* c, const Box& b, const Prim& pr, const FaceFlux& out, int l_lo, int l_cnt) {
+    const bool vec = xpair_vec(b, pr, out), ppm = c->recon == CUMC_PPMC;
+    auto go = [&](auto kern) {
+        launch_grid(c, CUMC_K_SWEEP_X, xpair_grid(b, l_cnt), XP_THREADS, 0, kern, b, c->tabs, pr, c->ggas, out, l_lo);
+    };
+    if (c->fast)
+        vec ? go(ppm ? k_sweep_xpair<4, double, true, true> : k_sweep_xpair<1, double, true, true>)
+            : go(ppm ? k_sweep_xpair<4, double, true, false> : k_sweep_xpair<1, double, true, false>);
+    else
+        vec ? go(ppm ? k_sweep_xpair<4, double, false, true> : k_sweep_xpair<1, double, false, true>)
+            : go(ppm ? k_sweep_xpair<4, double, false, false> : k_sweep_xpair<1, double, false, false>);
+}
+
 // l_lo, l_cnt: the z planes whose x rows (DIR 0) or y columns (DIR 1) the
 // default kernels sweep (l_cnt < 0: all); the other forms sweep everything
 template <int DIR>
@@ -278,7 +293,11 @@ void sweep(cumc_ctx* c, const Box& b, const Prim& pr, int l_lo = 0, int l_cnt = 
         }
         return;
     }
-    if (DIR == 0 && (mode == 0 || mode == 6)) {  // x: one lane per cell
+    if (DIR == 0 && mode == 0) {  // x: two cells a lane
+        sweep_xpair(c, b, pr, out, l_cnt >= 0 ? l_lo : 0, l_cnt >= 0 ? l_cnt : b.nz + 2);
+        return;
+    }
+    if (DIR == 0 && mode == 6) {  // x: one lane per cell
         const int cnt = l_cnt >= 0 ? l_cnt : b.nz + 2, lo = l_cnt >= 0 ? l_lo : 0;
         const bool ppm = c->recon == CUMC_PPMC;
         if (c->fast)
@@ -314,6 +333,13 @@ int sweep_attributes(cumc_ctx* c) {
     for (const void* f : k) {
         cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw_smem<double>());
         if (e != cudaSuccess) return cuda_fail(c, e, "cudaFuncSetAttribute(sweep smem)");
+    }
+    const void* m[9] = {(const void*)k_emf_ct<1, 1>, (const void*)k_emf_ct<1, 2>, (const void*)k_emf_ct<1, 3>,
+                        (const void*)k_emf_ct<2, 1>, (const void*)k_emf_ct<2, 2>, (const void*)k_emf_ct<2, 3>,
+                        (const void*)k_emf_ct<3, 1>, (const void*)k_emf_ct<3, 2>, (const void*)k_emf_ct<3, 3>};
+    for (const void* f : m) {
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EmfCtSmem));
+        if (e != cudaSuccess) return cuda_fail(c, e, "cudaFuncSetAttribute(EMF tile smem)");
     }
     return CUMC_OK;
 }

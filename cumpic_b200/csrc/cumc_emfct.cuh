@@ -20,10 +20,12 @@
 
 namespace cumc {
 
-constexpr int EC_TX = 32, EC_TY = 8;           // face triples of a tile
+#ifndef CUMC_EC_TY
+#define CUMC_EC_TY 8
+#endif
+constexpr int EC_TX = 32, EC_TY = CUMC_EC_TY;  // face triples of a tile
 constexpr int EC_CX = EC_TX + 2, EC_CY = EC_TY + 2;  // cells j0-1..j0+32, k0-1..k0+8
 constexpr int EC_EX = EC_TX + 1, EC_EY = EC_TY + 1;  // edges j0-1..j0+31, k0-1..k0+7
-constexpr int EC_SEG = 32;                     // planes a block marches over (at most; emf_ct_grid)
 
 // shared memory of a tile; R is the EMFs' type (double, or float in the
 // mixed form)
@@ -145,6 +147,40 @@ __device__ __forceinline__ void ec_edge_finish(const Box& b, EmfCtSmemT<R>& S, c
     S.ez[ek][ej] = ez;
 }
 
+// ct_lrk (solver/mhd.f90:137-148) from the nine edge EMFs around a face triple:
+// the six quotients of ct_lrk, bit for bit, through quot_group (on Cartesian
+// grids two share each width)
+template <int COORD>
+__device__ __forceinline__ void ct_curl(const CTf& g, double Ex, double Ex_lm, double Ex_km, double Ey, double Ey_lm,
+                                        double Ey_jm, double Ez, double Ez_km, double Ez_jm, double (&L)[3]) {
+    const double nxz = Ez * g.bx_ez_p - Ez_km * g.bx_ez_m, nxy = Ey * g.bx_ey_p - Ey_lm * g.bx_ey_m;
+    const double nyx = Ex * g.by_ex_p - Ex_lm * g.by_ex_m, nyz = Ez * g.by_ez_p - Ez_jm * g.by_ez_m;
+    const double nzy = Ey * g.bz_ey_p - Ey_jm * g.bz_ey_m, nzx = Ex * g.bz_ex_p - Ex_km * g.bz_ex_m;
+    double qx[2], qy[2], qz[2];  // by the widths along x, y, z
+    if constexpr (COORD == 1) {
+        const double ax[2] = {nyz, nzy}, ay[2] = {nxz, nzx}, az[2] = {nxy, nyx};
+        quot_group(ax, g.by_ez_c, qx);
+        quot_group(ay, g.bx_ez_c, qy);
+        quot_group(az, g.bx_ey_c, qz);
+    } else {
+        auto one = [](double a, double b) {
+            const double n[1] = {a};
+            double q[1];
+            quot_group(n, b, q);
+            return q[0];
+        };
+        qx[0] = one(nyz, g.by_ez_c);
+        qx[1] = one(nzy, g.bz_ey_c);
+        qy[0] = one(nxz, g.bx_ez_c);
+        qy[1] = one(nzx, g.bz_ex_c);
+        qz[0] = one(nxy, g.bx_ey_c);
+        qz[1] = one(nyx, g.by_ex_c);
+    }
+    L[0] = -(qy[0] - qz[0]);
+    L[1] = -(qz[1] - qx[0]);
+    L[2] = -(qx[1] - qy[1]);
+}
+
 // Per plane a thread first issues its global loads (the flux half of its
 // edges, u_old and u of its face triple, the cell fields of its cells of the
 // next plane), so that one memory latency a plane is exposed instead of
@@ -205,9 +241,7 @@ __global__ void __launch_bounds__(EC_TX * EC_TY, CUMC_EC_MINB) k_emf_ct(Box b, T
             CTf g;
             geom_ct<COORD>(T, j, k, l, g);
             double L[3];
-            L[0] = -((Ez * g.bx_ez_p - Ez_km * g.bx_ez_m) / g.bx_ez_c - (Ey * g.bx_ey_p - Ey_lm * g.bx_ey_m) / g.bx_ey_c);
-            L[1] = -((Ex * g.by_ex_p - Ex_lm * g.by_ex_m) / g.by_ex_c - (Ez * g.by_ez_p - Ez_jm * g.by_ez_m) / g.by_ez_c);
-            L[2] = -((Ey * g.bz_ey_p - Ey_jm * g.bz_ey_m) / g.bz_ey_c - (Ex * g.bz_ex_p - Ex_km * g.bz_ex_m) / g.bz_ex_c);
+            ct_curl<COORD>(g, Ex, Ex_lm, Ex_km, Ey, Ey_lm, Ey_jm, Ez, Ez_km, Ez_jm, L);
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const double r = rk_point<STAGE>(u0v[c], ucv[c], dt, L[c]);
@@ -218,16 +252,25 @@ __global__ void __launch_bounds__(EC_TX * EC_TY, CUMC_EC_MINB) k_emf_ct(Box b, T
     }
 }
 
-// grid of a tiled EMF + CT launch and the planes a block marches over: 32,
-// halved (down to 4) while the grid would not fill `slots` resident blocks
-// twice (small boxes: the 128^3 adjoint box, the torus); each segment repeats
-// one plane of cell and edge EMFs
+// Grid of a tiled EMF + CT launch and the planes a block marches over: the
+// segment length that makes (rounds of `slots` resident blocks) x (planes + 1)
+// least; each segment repeats one plane of cell and edge EMFs. Against 32 planes
+// halved down to 4 (and the plain quotients in the curl): 192x128x64 torus 0.129
+// -> 0.115 ms, the 90x26x75 one 0.029 -> 0.019, a 512x4x4 tube 0.020 -> 0.011,
+// 256^3 0.73 -> 0.72.
 inline dim3 emf_ct_grid(const Box& b, long long slots, int* seg) {
     const unsigned gx = (unsigned)((b.nx + 1 + EC_TX - 1) / EC_TX), gy = (unsigned)((b.ny + 1 + EC_TY - 1) / EC_TY);
-    int s = EC_SEG;
-    while (s > 4 && (long long)gx * gy * ((b.nz + 1 + s - 1) / s) < 2 * slots) s /= 2;
-    *seg = s;
-    return dim3(gx, gy, (unsigned)((b.nz + 1 + s - 1) / s));
+    const int planes = b.nz + 1;
+    long long best = -1;
+    for (int n = 1; n <= planes; ++n) {
+        const int s = (planes + n - 1) / n;
+        const long long rounds = ((long long)gx * gy * ((planes + s - 1) / s) + slots - 1) / slots;
+        if (best < 0 || rounds * (s + 1) < best) {
+            best = rounds * (s + 1);
+            *seg = s;
+        }
+    }
+    return dim3(gx, gy, (unsigned)((planes + *seg - 1) / *seg));
 }
 
 }  // namespace cumc

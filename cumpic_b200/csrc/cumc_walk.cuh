@@ -54,27 +54,33 @@ struct WalkGeom {
     }
 };
 
-// faces per segment: segments of near-equal length close to `target`
-inline int walk_segment(int faces, int target, int* nseg) {
-    int n = (faces + target - 1) / target;
-    if (n < 1) n = 1;
-    *nseg = n;
-    return (faces + n - 1) / n;
-}
-
-// segments of a walk along DIR over `ncols` columns: about 64 faces each,
-// shorter (down to 8) while the grid would give fewer than 32 warps per SM,
-// so that small boxes (a 128^3 adjoint box, the torus) still fill the GPU.
-// Each segment repeats the walk's prologue (three slopes, two interface
-// values, one fix a field), a few per cent of a face's work at 8 faces.
+// Segments of a walk along DIR over `ncols` columns. Equal blocks run in
+// rounds of the WK_RESIDENT blocks a SM that fit (96 registers and 21.5 KB of
+// shared memory a 64-thread block), and a segment costs its faces plus a
+// prologue (three slopes, two interface values and a fix a field, and a
+// memory latency: about one and a half faces), so the count is taken that
+// makes rounds x (faces + 1.5) least. Against about 64 faces, halved down to
+// 8 while the grid gave fewer than 32 warps a SM: 64^3 0.036 -> 0.029 ms a
+// walk, the 90x26x75 torus 0.029 -> 0.023, a 512x4x4 tube 0.021 -> 0.013; 256^3
+// unchanged (0.90).
+constexpr int WK_RESIDENT = 10;
 template <int DIR>
 inline int walk_segment_for(const Box& b, long long ncols, int sm_count, int* nseg) {
     const int faces = WalkGeom<DIR>::nd(b) + 1;
-    const long long blocks = (ncols + WK_THREADS - 1) / WK_THREADS;
-    const long long want = (long long)sm_count * 32 / (WK_THREADS / 32);  // blocks for 32 warps per SM
-    int target = 64;
-    while (target > 8 && blocks * ((faces + target - 1) / target) < want) target /= 2;
-    return walk_segment(faces, target, nseg);
+    const long long blocks = (ncols + WK_THREADS - 1) / WK_THREADS, slots = (long long)sm_count * WK_RESIDENT;
+    long long best = -1;
+    int best_seg = faces;
+    for (int n = 1; n <= faces; ++n) {
+        const int seg = (faces + n - 1) / n;
+        const long long rounds = (blocks * ((faces + seg - 1) / seg) + slots - 1) / slots;
+        const long long cost = rounds * (2 * seg + 3);
+        if (best < 0 || cost < best) {
+            best = cost;
+            best_seg = seg;
+        }
+    }
+    *nseg = (faces + best_seg - 1) / best_seg;
+    return best_seg;
 }
 
 // cell index 0 (along DIR) of column `col` of the block's grid, clamped to
@@ -495,6 +501,128 @@ __global__ void __launch_bounds__(128, CUMC_XWARP_MINB) k_sweep_xwarp(Box b, Tab
 
 inline long long xwarp_threads(const Box& b, int l_cnt = -1) {
     return (long long)(b.ny + 2) * (l_cnt < 0 ? b.nz + 2 : l_cnt) * ((b.nx + 1 + XW_FACES - 1) / XW_FACES) * 32;
+}
+
+// ---------------------------------------------------------------------------
+// x sweep with two cells a lane (the default in FP64). The rows 0:n+1 of a plane are
+// taken as one line of SX (ny + 2) cells: a warp holds 64 consecutive cells of
+// it, lane i the cells 2i and 2i+1, forms each cell's slope, interface value
+// and extremum fix once (five shuffled values a field and two cells, against
+// eight in k_sweep_xwarp) and solves HLL at 58 faces, so that 58 of 64 lanes'
+// work counts instead of 27 of 32, and a row that is no multiple of 27 faces
+// costs nothing but its five faces that straddle the row's end, which are
+// skipped. The pair's states wait in shared memory between the reconstruction
+// and the two solves (one body, run twice), which keeps the registers to the
+// walkers' 96. VEC: with SX even a pair starts on a 16-byte boundary (8 bytes
+// in FP32) and moves as one vector.
+// ---------------------------------------------------------------------------
+constexpr int XP_FACES = 58, XP_THREADS = 128;
+#ifndef CUMC_XPAIR_MINB
+#define CUMC_XPAIR_MINB 5
+#endif
+template <typename R>
+struct Pair {
+    R a, b;
+};
+template <bool VEC, typename R>
+__device__ __forceinline__ Pair<R> ld_pair(const R* p, int i) {
+    if constexpr (VEC) {
+        static_assert(sizeof(R) == 8, "FP64 pairs");
+        const double2 v = *reinterpret_cast<const double2*>(p + i);
+        return {v.x, v.y};
+    } else {
+        return {p[i], p[i + 1]};
+    }
+}
+template <bool VEC, typename R>
+__device__ __forceinline__ void st_pair(R* p, int i, R a, R b, bool oka, bool okb) {
+    if (VEC && oka && okb) {
+        *reinterpret_cast<double2*>(p + i) = make_double2(a, b);
+    } else {
+        if (oka) p[i] = a;
+        if (okb) p[i + 1] = b;
+    }
+}
+
+template <int RECON, typename R, bool RECIP, bool VEC>
+__global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box b, Tabs T, PrimT<R> pr, R ggas,
+                                                                           FaceFluxT<R> out, int l_lo) {
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ R sm[28][XP_THREADS];  // states of the pair's two faces: left 7, right 7 each
+    const int cells = b.SX * (b.ny + 2);
+    const int w = blockIdx.x * (XP_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31, tid = threadIdx.x;
+    if (w * XP_FACES + 2 >= cells || (b.skip && *b.skip)) return;  // uniform over the warp
+    const int m = w * XP_FACES + 2 * lane;  // position of the lane's first cell in the plane's line
+    const int g = b.idx(-2, 0, l_lo + (int)blockIdx.y) + m;
+    const int j0 = m % b.SX - 2, j1 = j0 == b.nx + 3 ? -2 : j0 + 1;
+    const bool faces = lane >= 1 && lane <= 29;
+    const bool ok0 = faces && m < cells && j0 >= 0 && j0 <= b.nx;
+    const bool ok1 = faces && m + 1 < cells && j1 >= 0 && j1 <= b.nx;
+    const AxisTabs A = T.ax[0];
+    const R* src[7] = {pr.w[0], pr.w[1], pr.w[2], pr.w[3], pr.w[4], pr.bc[1], pr.bc[2]};
+#pragma unroll
+    for (int v = 0; v < 7; ++v) {
+        const Pair<R> x = ld_pair<VEC>(src[v], g);
+        const R xm = __shfl_up_sync(FULL, x.b, 1), xp = __shfl_down_sync(FULL, x.a, 1);
+        R vm0, vp0, vm1, vp1;
+        if (RECON == 4) {
+            const R d0 = ppm_slope(xm, x.a, x.b, (R)A.s0[j0], (R)A.s1[j0]);
+            const R d1 = ppm_slope(x.a, x.b, xp, (R)A.s0[j1], (R)A.s1[j1]);
+            const R d2 = __shfl_down_sync(FULL, d0, 1);
+            const R V0 = ppm_face(x.a, x.b, d0, d1, (R)A.a0[j0], (R)A.a1[j0], (R)A.a2[j0], (R)A.a3[j0]);
+            const R V1 = ppm_face(x.b, xp, d1, d2, (R)A.a0[j1], (R)A.a1[j1], (R)A.a2[j1], (R)A.a3[j1]);
+            const R Vm = __shfl_up_sync(FULL, V1, 1);
+            ppm_fix(x.a, Vm, V0, vm0, vp0);
+            ppm_fix(x.b, V0, V1, vm1, vp1);
+        } else {
+            const R s0 = tvd_slope(xm, x.a, x.b, (R)A.tcf[j0], (R)A.tcb[j0]);
+            const R s1 = tvd_slope(x.a, x.b, xp, (R)A.tcf[j1], (R)A.tcb[j1]);
+            vm0 = x.a - R(0.5) * s0;
+            vp0 = x.a + R(0.5) * s0;
+            vm1 = x.b - R(0.5) * s1;
+            vp1 = x.b + R(0.5) * s1;
+        }
+        sm[v][tid] = vp0;  // face 2i | 2i+1: vp_out of its left cell, vm_out of its right cell
+        sm[7 + v][tid] = vm1;
+        sm[14 + v][tid] = vp1;
+        sm[21 + v][tid] = __shfl_down_sync(FULL, vm0, 1);
+    }
+    if (!ok0 && !ok1) return;
+    const Pair<R> bn = ld_pair<VEC>(pr.bf[0], g);
+    R fx[7];
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f) {
+        if (f == 0 ? ok0 : ok1) {
+            constexpr int slot[7] = {IRHO, IVX, IVY, IVZ, ITAU, IBY, IBZ};
+            R wl[8], wr[8];
+#pragma unroll
+            for (int v = 0; v < 7; ++v) {
+                wl[slot[v]] = sm[14 * f + v][tid];
+                wr[slot[v]] = sm[14 * f + 7 + v][tid];
+            }
+            wl[IBX] = wr[IBX] = f == 0 ? bn.a : bn.b;
+            sweep_hll<0, R, RECIP>(wl, wr, ggas, fx);
+        }
+        if (f == 0) {
+#pragma unroll
+            for (int i = 0; i < 7; ++i) sm[i][tid] = fx[i];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 7; ++i) st_pair<VEC>(out.f[i], g, sm[i][tid], fx[i], ok0, ok1);
+}
+
+// the vector form's conditions: every pair aligned to its own size
+template <typename R>
+inline bool xpair_vec(const Box& b, const PrimT<R>& pr, const FaceFluxT<R>& out) {
+    uintptr_t at = (uintptr_t)pr.bc[1] | (uintptr_t)pr.bc[2] | (uintptr_t)pr.bf[0];
+    for (int q = 0; q < 5; ++q) at |= (uintptr_t)pr.w[q];
+    for (int q = 0; q < 7; ++q) at |= (uintptr_t)out.f[q];
+    return b.SX % 2 == 0 && at % (2 * sizeof(R)) == 0;
+}
+inline dim3 xpair_grid(const Box& b, int l_cnt) {
+    const int warps = (b.SX * (b.ny + 2) - 2 + XP_FACES - 1) / XP_FACES;
+    return dim3((unsigned)((warps + XP_THREADS / 32 - 1) / (XP_THREADS / 32)), (unsigned)l_cnt);
 }
 
 }  // namespace cumc
