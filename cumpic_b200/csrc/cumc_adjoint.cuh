@@ -46,108 +46,25 @@ struct AdjPrim {
 // reconstruction transposes (branches frozen by recomputation)
 // ---------------------------------------------------------------------------
 
-// ppm_slope's value (bit-identical: the same expression) and its partial
-// derivatives with respect to (vm, vc, vp), on the branch the value took
-struct SlopeGrad {
-    double d, gm, gc, gp;
-};
-__device__ __forceinline__ SlopeGrad ppm_slope_grad(double vm, double vc, double vp, double b0, double b1) {
-    SlopeGrad s{0.0, 0.0, 0.0, 0.0};
-    const double delta = b0 * (vp - vc) + b1 * (vc - vm);
-    if ((vp - vc) * (vc - vm) > 0.0) {
-        const double m1 = fabs(delta), m2 = 2.0 * fabs(vc - vm), m3 = 2.0 * fabs(vc - vp);
-        const double sd = copysign(1.0, delta);
-        const double m12 = fmin(m1, m2);
-        s.d = fmin(m12, m3) * sd;
-        if (m12 <= m3 && m1 <= m2) {  // slope = delta
-            s.gm = -b1;
-            s.gc = b1 - b0;
-            s.gp = b0;
-        } else if (m12 <= m3) {  // slope = sd 2 |vc - vm|
-            const double g = sd * 2.0 * copysign(1.0, vc - vm);
-            s.gm = -g;
-            s.gc = g;
-        } else {  // slope = sd 2 |vc - vp|
-            const double g = sd * 2.0 * copysign(1.0, vc - vp);
-            s.gc = g;
-            s.gp = -g;
-        }
-    }
-    return s;
-}
-
-// transpose of the reconstruction of one cell from v[0..4] = cells c-2..c+2:
-// seeds lvm, lvp on (vm_out, vp_out); adds to lv[0..4]
-template <int RECON>
-__device__ __forceinline__ void recon_adj(const AxisTabs& A, int c, const double v[5], double lvm, double lvp,
-                                          double lv[5]) {
+// transpose of the TVD reconstruction of one cell from v[1..3] = cells
+// c-1..c+1: seeds lvm, lvp on (vm_out, vp_out); adds to lv[1..3]
+__device__ __forceinline__ void tvd_adj(const AxisTabs& A, int c, const double v[5], double lvm, double lvp,
+                                        double lv[5]) {
     if (lvm == 0.0 && lvp == 0.0) return;
-    if (RECON == 4) {
-        const SlopeGrad sm = ppm_slope_grad(v[0], v[1], v[2], A.s0[c - 1], A.s1[c - 1]);
-        const SlopeGrad sc = ppm_slope_grad(v[1], v[2], v[3], A.s0[c], A.s1[c]);
-        const SlopeGrad sp = ppm_slope_grad(v[2], v[3], v[4], A.s0[c + 1], A.s1[c + 1]);
-        const double dmm = sm.d, dmc = sc.d, dmp = sp.d;
-        const double vl = ppm_face(v[1], v[2], dmm, dmc, A.a0[c - 1], A.a1[c - 1], A.a2[c - 1], A.a3[c - 1]);
-        const double vr = ppm_face(v[2], v[3], dmc, dmp, A.a0[c], A.a1[c], A.a2[c], A.a3[c]);
-        const double vc = v[2];
-        // ppm_fix transpose
-        double lvc = 0.0, lvl = 0.0, lvr = 0.0;
-        if ((vr - vc) * (vc - vl) <= 0.0) {
-            lvc += lvm + lvp;
-        } else {
-            double vm1 = vl;
-            if ((vr - vl) * ((vl - 3.0 * vc) + 2.0 * vr) < 0.0) {
-                vm1 = 3.0 * vc - 2.0 * vr;
-                lvc += 3.0 * lvm;
-                lvr -= 2.0 * lvm;
-            } else {
-                lvl += lvm;
-            }
-            if ((vr - vm1) * ((3.0 * vc - 2.0 * vl) - vr) < 0.0) {
-                lvc += 3.0 * lvp;
-                lvl -= 2.0 * lvp;
-            } else {
-                lvr += lvp;
-            }
-        }
-        // interface values: V = vc' + (a0 + a1)(vp' - vc') + a2 dmp' + a3 dmc'
-        double ldmm = 0.0, ldmc = 0.0, ldmp = 0.0;
-        {
-            const double s = A.a0[c - 1] + A.a1[c - 1];
-            lv[1] += (1.0 - s) * lvl;
-            lv[2] += s * lvl;
-            ldmc += A.a2[c - 1] * lvl;
-            ldmm += A.a3[c - 1] * lvl;
-        }
-        {
-            const double s = A.a0[c] + A.a1[c];
-            lv[2] += (1.0 - s) * lvr;
-            lv[3] += s * lvr;
-            ldmp += A.a2[c] * lvr;
-            ldmc += A.a3[c] * lvr;
-        }
-        lv[2] += lvc;
-        lv[0] += ldmm * sm.gm;
-        lv[1] += ldmm * sm.gc + ldmc * sc.gm;
-        lv[2] += ldmm * sm.gp + ldmc * sc.gc + ldmp * sp.gm;
-        lv[3] += ldmc * sc.gp + ldmp * sp.gc;
-        lv[4] += ldmp * sp.gp;
-    } else {
-        // vm = vc - sl/2, vp = vc + sl/2, sl = minmod of dqf = 2(vp-vc)/cf, dqb = 2(vc-vm)/cb
-        lv[2] += lvm + lvp;
-        const double lsl = 0.5 * (lvp - lvm);
-        const double cf = A.tcf[c], cb = A.tcb[c];
-        const double dqf = (2.0 * (v[3] - v[2])) / cf;
-        const double dqb = (2.0 * (v[2] - v[1])) / cb;
-        const double sf = copysign(1.0, dqf), sb = copysign(1.0, dqb);
-        if (sf != sb) return;  // slope 0
-        if (fabs(dqf) <= fabs(dqb)) {  // slope = dqf
-            lv[3] += 2.0 * lsl / cf;
-            lv[2] -= 2.0 * lsl / cf;
-        } else {  // slope = dqb
-            lv[2] += 2.0 * lsl / cb;
-            lv[1] -= 2.0 * lsl / cb;
-        }
+    // vm = vc - sl/2, vp = vc + sl/2, sl = minmod of dqf = 2(vp-vc)/cf, dqb = 2(vc-vm)/cb
+    lv[2] += lvm + lvp;
+    const double lsl = 0.5 * (lvp - lvm);
+    const double cf = A.tcf[c], cb = A.tcb[c];
+    const double dqf = (2.0 * (v[3] - v[2])) / cf;
+    const double dqb = (2.0 * (v[2] - v[1])) / cb;
+    const double sf = copysign(1.0, dqf), sb = copysign(1.0, dqb);
+    if (sf != sb) return;  // slope 0
+    if (fabs(dqf) <= fabs(dqb)) {  // slope = dqf
+        lv[3] += 2.0 * lsl / cf;
+        lv[2] -= 2.0 * lsl / cf;
+    } else {  // slope = dqb
+        lv[2] += 2.0 * lsl / cb;
+        lv[1] -= 2.0 * lsl / cb;
     }
 }
 
@@ -160,9 +77,9 @@ struct SideAdj {
     // the forward's divisions (no branch depends on them)
     double rho, irho, v[3], p, b[3], e, vsq, bsq, E, hb2, vdotb;
     double Lrho, Lv[3], Lp, Lb[3], LE, Lhb2, Lvdotb;
-    __device__ __forceinline__ void init(const double w[8], double ig1) {
+    __device__ __forceinline__ void init(const double w[8], double irho_, double ig1) {
         rho = w[IRHO];
-        irho = 1.0 / rho;
+        irho = irho_;
         v[0] = w[IVX]; v[1] = w[IVY]; v[2] = w[IVZ];
         p = w[ITAU];
         b[0] = w[IBX]; b[1] = w[IBY]; b[2] = w[IBZ];
@@ -249,117 +166,149 @@ struct SideAdj {
     }
 };
 
-// adjoint of cf = signalspeed(cs, bn, bt1, bt2, rho): adds to the arguments' adjoints
-__device__ __forceinline__ void signalspeed_adj(double cs, double bn, double bt1, double bt2, double rho, double cf,
-                                                double lcf, double& lcs, double& lbn, double& lbt1, double& lbt2,
-                                                double& lrho) {
-    if (lcf == 0.0 || !(cf > 0.0)) return;
-    const double irho = 1.0 / rho;
-    const double a2 = cs * cs;
-    const double b2n = (bn * bn) * irho, b2t1 = (bt1 * bt1) * irho, b2t2 = (bt2 * bt2) * irho;
-    const double b2 = (b2n + b2t1) + b2t2;
-    const double inner = ((a2 * a2 + b2 * b2) + (2.0 * b2) * a2) - (4.0 * a2) * b2n;
-    const double lsum = lcf * 0.25 / cf;  // d cf / d (a2 + b2 + s)
-    double la2 = lsum, lb2 = lsum, lb2n = 0.0;
-    if (inner > 0.0) {
-        const double ls = lsum * 0.5 / sqrt(inner);  // d sqrt(inner) / d inner
-        la2 += ls * (2.0 * (a2 + b2) - 4.0 * b2n);
-        lb2 += ls * 2.0 * (a2 + b2);
-        lb2n += ls * (-4.0 * a2);
+// one side's speeds as the forward has them (bit for bit, so that the branches
+// below are the forward's), and the reciprocals that weight derivatives
+template <int DIR>
+struct SideWave {
+    double irho, cs, cf, sq, ics_p;  // 1/rho, sound and fast speed, sqrt(rho), 1/p
+    double a2, b2n, b2, is, icf;     // of compute_signalspeed; is = 1/sqrt(inner) or 0, icf = 1/cf
+};
+template <int DIR, bool ROUNDED>
+__device__ __forceinline__ SideWave<DIR> side_wave(const double (&w)[8], double g) {
+    constexpr int ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
+    const double rho = w[IRHO], p = w[ITAU];
+    SideWave<DIR> s;
+    double inner, root;
+    if constexpr (ROUNDED) {
+        const Recip r = recip_of(rho);
+        s.irho = r.y;
+        s.cs = root_of(quot(g * p, rho, r));
+        s.a2 = s.cs * s.cs;
+        s.b2n = quot(w[ibn] * w[ibn], rho, r);
+        s.b2 = (s.b2n + quot(w[ibt1] * w[ibt1], rho, r)) + quot(w[ibt2] * w[ibt2], rho, r);
+        inner = __fma_rn(-4.0, s.a2 * s.b2n, __fma_rn(2.0, s.b2 * s.a2, s.a2 * s.a2 + s.b2 * s.b2));
+        root = root_pos(inner);
+        s.cf = root_of(0.5 * ((s.a2 + s.b2) + root));
+        s.sq = root_of(rho);
+        s.is = inner > 0.0 ? recip_r(root) : 0.0;
+        s.icf = recip_r(s.cf);
+        s.ics_p = recip_r(p);
+    } else {
+        s.irho = 1.0 / rho;
+        s.cs = sqrt((g * p) / rho);
+        s.a2 = s.cs * s.cs;
+        s.b2n = (w[ibn] * w[ibn]) / rho;
+        s.b2 = (s.b2n + (w[ibt1] * w[ibt1]) / rho) + (w[ibt2] * w[ibt2]) / rho;
+        inner = ((s.a2 * s.a2 + s.b2 * s.b2) + (2.0 * s.b2) * s.a2) - (4.0 * s.a2) * s.b2n;
+        root = sqrt(fmax(inner, 0.0));
+        s.cf = sqrt(0.5 * ((s.a2 + s.b2) + root));
+        s.sq = sqrt(rho);
+        s.is = inner > 0.0 ? 1.0 / root : 0.0;
+        s.icf = s.cf > 0.0 ? 1.0 / s.cf : 0.0;
+        s.ics_p = s.cs > 0.0 ? 1.0 / p : 0.0;
     }
-    lb2n += lb2;
-    lcs += 2.0 * cs * la2;
-    lbn += 2.0 * bn * irho * lb2n;
-    lbt1 += 2.0 * bt1 * irho * lb2;
-    lbt2 += 2.0 * bt2 * irho * lb2;
-    lrho -= (b2n * lb2n + (b2t1 + b2t2) * lb2) * irho;
+    return s;
+}
+// the plain form, for densities and pressures outside the rounded one's range
+template <int DIR>
+__device__ __noinline__ SideWave<DIR> side_wave_plain(const double* wp, double g) {
+    double w[8];
+    for (int q = 0; q < 8; ++q) w[q] = wp[q];
+    return side_wave<DIR, false>(w, g);
 }
 
-// adjoint of out[7] = hll_flux7<DIR>(wl, wr): lout[7] -> lwl[8], lwr[8] (added)
-template <int DIR>
-__device__ __forceinline__ void hll_adj(const double wl[8], const double wr[8], double g, const double lout[7],
-                                        double lwl[8], double lwr[8]) {
+// Adjoint of out[7] = hll_flux7<DIR>(wl, wr): lout[7] -> put(side, out[8]), called
+// once a side. With id = 1/(sR - sL) and ln = lout id, the wave speeds enter
+// the HLL average only through the jumps dF = sum ln (fR - fL) and
+// dU = sum ln (uR - uL): d/dsL = id sR (sR dU - dF), d/dsR = id sL (dF - sL dU). So the
+// two sides are transposed one after the other, each with ln scaled by its two
+// coefficients, and only one side's adjoints are live at a time.
+template <int DIR, typename Put>
+__device__ __forceinline__ void hll_adj(const double (&wl)[8], const double (&wr)[8], double g, const double (&lout)[7],
+                                        Put&& put) {
     constexpr int ivn = IVX + DIR;
-    constexpr int ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
     constexpr int bt_a = DIR == 0 ? IBY : IBX;
     constexpr int bt_b = DIR == 2 ? IBY : IBZ;
-    const int comp[7] = {IRHO, IVX, IVY, IVZ, ITAU, bt_a, bt_b};
-    const double ig1 = 1.0 / (g - 1.0);
-    SideAdj<DIR> L, R;
-    L.init(wl, ig1);
-    R.init(wr, ig1);
-    const double csL = sqrt((g * wl[ITAU]) / wl[IRHO]);
-    const double csR = sqrt((g * wr[ITAU]) / wr[IRHO]);
-    const double cfL = signalspeed(csL, wl[ibn], wl[ibt1], wl[ibt2], wl[IRHO]);
-    const double cfR = signalspeed(csR, wr[ibn], wr[ibt1], wr[ibt2], wr[IRHO]);
-    const double sqL = sqrt(wl[IRHO]), sqR = sqrt(wr[IRHO]);
-    const double ubar = roe_avg(wl[ivn], wr[ivn], sqL, sqR);
-    const double cbar = roe_avg(cfL, cfR, sqL, sqR);
-    const double aL = wl[ivn] - cfL, bL = ubar - cbar;
-    const double aR = wr[ivn] + cfR, bR = ubar + cbar;
-    const double sL = fmin(aL, bL), sR = fmax(aR, bR);
-    double lsL = 0.0, lsR = 0.0;
-    if (sL >= 0.0) {
+    constexpr int comp[7] = {IRHO, IVX, IVY, IVZ, ITAU, bt_a, bt_b};
+    const double ig1 = recip_r(g - 1.0);
+    SideWave<DIR> w[2];
+    if (range_max(wl[IRHO], range_max(wr[IRHO], range_max(wl[ITAU], range_max(wr[ITAU], 0u)))) < RANGE_SPAN) {
+        w[0] = side_wave<DIR, true>(wl, g);
+        w[1] = side_wave<DIR, true>(wr, g);
+    } else {
+        double c[8];
 #pragma unroll
-        for (int c = 0; c < 7; ++c) L.f_adj(comp[c], lout[c]);
-    } else if (sL <= 0.0 && sR >= 0.0) {
-        const double id = 1.0 / (sR - sL);
-        double ld = 0.0;
+        for (int q = 0; q < 8; ++q) c[q] = wl[q];
+        w[0] = side_wave_plain<DIR>(c, g);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) c[q] = wr[q];
+        w[1] = side_wave_plain<DIR>(c, g);
+    }
+    const double sqs = w[0].sq + w[1].sq;
+    const Recip rs = recip_of(sqs);
+    const double ubar = quot(w[0].sq * wl[ivn] + w[1].sq * wr[ivn], sqs, rs);
+    const double cbar = quot(w[0].sq * w[0].cf + w[1].sq * w[1].cf, sqs, rs);
+    const double aL = wl[ivn] - w[0].cf, bL = ubar - cbar;
+    const double aR = wr[ivn] + w[1].cf, bR = ubar + cbar;
+    const double sL = fmin(aL, bL), sR = fmax(aR, bR);
+    double ln[7], kf[2], ku[2], lsL = 0.0, lsR = 0.0;
+    const bool mid = !(sL >= 0.0) && sR >= 0.0;
+    const double id = mid ? recip_r(sR - sL) : 1.0;
+#pragma unroll
+    for (int c = 0; c < 7; ++c) ln[c] = lout[c] * id;
+    kf[0] = mid ? sR : sL >= 0.0 ? 1.0 : 0.0;
+    kf[1] = mid ? -sL : sL >= 0.0 ? 0.0 : 1.0;
+    ku[1] = mid ? sL * sR : 0.0;
+    ku[0] = -ku[1];
+    if (mid) {
+        SideAdj<DIR> L, R;
+        L.init(wl, w[0].irho, ig1);
+        R.init(wr, w[1].irho, ig1);
+        double dF = 0.0, dU = 0.0;
 #pragma unroll
         for (int c = 0; c < 7; ++c) {
-            const int q = comp[c];
-            const double fl = L.f(q), fr = R.f(q), ul = L.u(q), ur = R.u(q);
-            const double out = ((sR * fl - sL * fr) + (sL * sR) * (ur - ul)) * id;
-            const double ln = lout[c] * id;
-            ld -= ln * out;
-            L.f_adj(q, sR * ln);
-            R.f_adj(q, -sL * ln);
-            R.u_adj(q, sL * sR * ln);
-            L.u_adj(q, -sL * sR * ln);
-            lsR += ln * (fl + sL * (ur - ul));
-            lsL += ln * (-fr + sR * (ur - ul));
+            dF += ln[c] * (R.f(comp[c]) - L.f(comp[c]));
+            dU += ln[c] * (R.u(comp[c]) - L.u(comp[c]));
         }
-        lsR += ld;
-        lsL -= ld;
-    } else {
+        lsL = id * sR * (sR * dU - dF);
+        lsR = id * sL * (dF - sL * dU);
+    }
+    // sL = min(aL, bL), sR = max(aR, bR), then the Roe averages
+    double lvn[2] = {0.0, 0.0}, lcf[2] = {0.0, 0.0}, lubar = 0.0, lcbar = 0.0;
+    if (aL <= bL) { lvn[0] += lsL; lcf[0] -= lsL; } else { lubar += lsL; lcbar -= lsL; }
+    if (aR >= bR) { lvn[1] += lsR; lcf[1] += lsR; } else { lubar += lsR; lcbar += lsR; }
+    lubar *= rs.y;
+    lcbar *= rs.y;
 #pragma unroll
-        for (int c = 0; c < 7; ++c) R.f_adj(comp[c], lout[c]);
+    for (int s = 0; s < 2; ++s) {
+        const double(&x)[8] = s == 0 ? wl : wr;
+        const SideWave<DIR>& v = w[s];
+        SideAdj<DIR> S;
+        S.init(x, v.irho, ig1);
+#pragma unroll
+        for (int c = 0; c < 7; ++c) {
+            S.f_adj(comp[c], kf[s] * ln[c]);
+            S.u_adj(comp[c], ku[s] * ln[c]);
+        }
+        const double lsq = lubar * (x[ivn] - ubar) + lcbar * (v.cf - cbar);
+        const double lc = lcf[s] + lcbar * v.sq;
+        S.Lv[DIR] += lvn[s] + lubar * v.sq;
+        S.Lrho += 0.5 * lsq * (v.sq * v.irho);  // d sqrt(rho) = d rho sqrt(rho)/(2 rho)
+        // cf = sqrt((a2 + b2 + sqrt(inner))/2): signalspeed's transpose
+        const double lsum = lc * 0.25 * v.icf, ls = lsum * 0.5 * v.is, ab = v.a2 + v.b2;
+        const double la2 = lsum + ls * (2.0 * ab - 4.0 * v.b2n), lb2 = lsum + ls * 2.0 * ab;
+        const double lb2n = lb2 - 4.0 * ls * v.a2;
+        S.Lb[DIR] += 2.0 * x[IBX + DIR] * v.irho * lb2n;
+        S.Lb[(DIR + 1) % 3] += 2.0 * x[IBX + (DIR + 1) % 3] * v.irho * lb2;
+        S.Lb[(DIR + 2) % 3] += 2.0 * x[IBX + (DIR + 2) % 3] * v.irho * lb2;
+        S.Lrho -= (v.b2n * lb2n + (v.b2 - v.b2n) * lb2) * v.irho;
+        // a2 = g p / rho
+        S.Lp += la2 * v.a2 * v.ics_p;
+        S.Lrho -= la2 * v.a2 * v.irho;
+        double out[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        S.finish(ig1, out);
+        put(s, out);
     }
-    // sL = min(aL, bL), sR = max(aR, bR)
-    double lvnL = 0.0, lvnR = 0.0, lcfL = 0.0, lcfR = 0.0, lubar = 0.0, lcbar = 0.0;
-    if (aL <= bL) { lvnL += lsL; lcfL -= lsL; } else { lubar += lsL; lcbar -= lsL; }
-    if (aR >= bR) { lvnR += lsR; lcfR += lsR; } else { lubar += lsR; lcbar += lsR; }
-    // Roe averages
-    const double iss = 1.0 / (sqL + sqR);
-    double lsqL = (lubar * (wl[ivn] - ubar) + lcbar * (cfL - cbar)) * iss;
-    double lsqR = (lubar * (wr[ivn] - ubar) + lcbar * (cfR - cbar)) * iss;
-    lvnL += lubar * sqL * iss;
-    lvnR += lubar * sqR * iss;
-    lcfL += lcbar * sqL * iss;
-    lcfR += lcbar * sqR * iss;
-    // fast speeds
-    double lcsL = 0.0, lcsR = 0.0;
-    signalspeed_adj(csL, wl[ibn], wl[ibt1], wl[ibt2], wl[IRHO], cfL, lcfL, lcsL, L.Lb[DIR], L.Lb[(DIR + 1) % 3],
-                    L.Lb[(DIR + 2) % 3], L.Lrho);
-    signalspeed_adj(csR, wr[ibn], wr[ibt1], wr[ibt2], wr[IRHO], cfR, lcfR, lcsR, R.Lb[DIR], R.Lb[(DIR + 1) % 3],
-                    R.Lb[(DIR + 2) % 3], R.Lrho);
-    // cs = sqrt(g p / rho): d cs = cs/2 (dp/p - drho/rho); sq = sqrt(rho): d sq = drho / (2 sq)
-    if (csL > 0.0) {
-        const double h = 0.5 * lcsL * csL;
-        L.Lp += h / wl[ITAU];
-        L.Lrho -= h * L.irho;
-    }
-    if (csR > 0.0) {
-        const double h = 0.5 * lcsR * csR;
-        R.Lp += h / wr[ITAU];
-        R.Lrho -= h * R.irho;
-    }
-    L.Lrho += 0.5 * lsqL / sqL;
-    R.Lrho += 0.5 * lsqR / sqR;
-    L.Lv[DIR] += lvnL;
-    R.Lv[DIR] += lvnR;
-    L.finish(ig1, lwl);
-    R.finish(ig1, lwr);
 }
 
 // ---------------------------------------------------------------------------
@@ -522,8 +471,11 @@ struct FaceAdj {
 // STATES form, one reconstruction per cell); each face reads its two states
 // and overwrites them with their adjoints. Otherwise the face reconstructs
 // its two cells itself.
+#ifndef CUMC_ADJ_MINB
+#define CUMC_ADJ_MINB 4
+#endif
 template <int COORD, int DIR, int RECON, bool FROM_STATES = false>
-__global__ void __launch_bounds__(128, 5) k_adj_hll(Box b, Tabs T, Prim pr, double ggas, AdjStage a, FaceAdj fa,
+__global__ void __launch_bounds__(128, CUMC_ADJ_MINB) k_adj_hll(Box b, Tabs T, Prim pr, double ggas, AdjStage a, FaceAdj fa,
                                                 double* lambf) {
     const int n0 = (DIR == 0 ? b.nx : b.nx + 1) + 1;
     const int n1 = (DIR == 1 ? b.ny : b.ny + 1) + 1;
@@ -633,14 +585,14 @@ __global__ void __launch_bounds__(128, 5) k_adj_hll(Box b, Tabs T, Prim pr, doub
     wl[IBX + DIR] = bn;
     wr[IBX + DIR] = bn;
 
-    double lwl[8] = {0, 0, 0, 0, 0, 0, 0, 0}, lwr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    hll_adj<DIR>(wl, wr, ggas, lf, lwl, lwr);
-    lambf[base] += lwl[IBX + DIR] + lwr[IBX + DIR];
+    double lbn = 0.0;
+    hll_adj<DIR>(wl, wr, ggas, lf, [&](int side, const double* out) {
+        lbn += out[IBX + DIR];
+        double* const* dst = side == 0 ? fa.l : fa.r;
 #pragma unroll
-    for (int v = 0; v < 7; ++v) {
-        fa.l[v][base] = lwl[slot[v]];
-        fa.r[v][base] = lwr[slot[v]];
-    }
+        for (int v = 0; v < 7; ++v) dst[v][base] = out[slot[v]];
+    });
+    lambf[base] += lbn;
 }
 
 // field v (0..6) of a sweep along DIR: source and adjoint arrays
@@ -657,10 +609,51 @@ __device__ __forceinline__ void sweep_field(const Prim& pr, const AdjPrim& o, in
     }
 }
 
+// The PPM reconstruction transpose, one slope, one interface value and one fix
+// a cell. The adjoint of the interface value between two cells is the sum of
+// the left one's vr and the right one's vl, so it is transposed once a face,
+// and a slope's adjoint (from its two faces) once a cell. A slope's derivatives
+// satisfy gc = -(gm + gp) on every branch.
+struct PpmSlope {
+    double d, gm, gp;
+};
+__device__ __forceinline__ PpmSlope ppm_slope_grad(double vm, double vc, double vp, double b0, double b1) {
+    const double up = vp - vc, dn = vc - vm;
+    const double delta = b0 * up + b1 * dn;
+    const double m1 = fabs(delta), hd = fabs(dn), hu = fabs(up);
+    const double m2 = 2.0 * hd, m3 = 2.0 * hu, m12 = min_mag(m1, m2);
+    const bool on = is_pos(up * dn);
+    const bool by_up = m12 > m3, by_dn = !by_up && m1 > m2;  // limited by 2 |vc - vp|, by 2 |vc - vm|
+    // sd 2 sign(dn); sign(up) = sign(dn) where the slope is on
+    const double g = copysign(2.0, delta) * copysign(1.0, dn);
+    PpmSlope s;
+    s.d = on ? copysign(min_mag(m12, m3), delta) : 0.0;
+    s.gm = !on || by_up ? 0.0 : by_dn ? -g : -b1;
+    s.gp = !on || by_dn ? 0.0 : by_up ? g : b0;
+    return s;
+}
+// ppm_fix's transpose at a cell with value vc and interface values vl, vr
+struct PpmFixAdj {
+    double c, l, r;
+};
+__device__ __forceinline__ PpmFixAdj ppm_fix_adj(double vc, double vl, double vr, double lvm, double lvp) {
+    const double c3 = 3.0 * vc;
+    const bool flat = !is_pos((vr - vc) * (vc - vl));
+    const bool t1 = is_neg((vr - vl) * __fma_rn(2.0, vr, vl - c3));
+    const double vm = t1 ? __fma_rn(-2.0, vr, c3) : vl;
+    const bool t2 = is_neg((vr - vm) * (__fma_rn(-2.0, vl, c3) - vr));
+    const double m1 = t1 ? lvm : 0.0, p1 = t2 ? lvp : 0.0;  // seeds that the fixes took over
+    PpmFixAdj a;
+    a.c = flat ? lvm + lvp : 3.0 * (m1 + p1);
+    a.l = flat ? 0.0 : (lvm - m1) - 2.0 * p1;
+    a.r = flat ? 0.0 : (lvp - p1) - 2.0 * m1;
+    return a;
+}
+
 // sweep^T, pass B along y or z: the reconstruction transpose. One thread
 // per (column, field, segment of RC_SEG cells) walks its segment: cell c's
 // reconstruction (vm_out, vp_out) took its seeds from faces c-1 and c; its
-// transpose adds to cells c-2..c+2, kept in a five-cell ring, and a cell is
+// transpose adds to cells c-2..c+2, kept in registers, and a cell is
 // complete once the walk has passed it by two. A segment writes cells
 // c0-2 .. c1+1, so the four cells next to each end of a segment also receive
 // from the neighbouring segment. The even segments run in one launch and
@@ -694,37 +687,96 @@ __global__ void __launch_bounds__(128) k_adj_recon_col(Box b, Tabs T, Prim pr, F
     auto emit = [&](int q, double val) {
         if (val != 0.0) dst[q * s] += val;
     };
-    double x[5] = {src[(c0 - 2) * s], src[(c0 - 1) * s], src[c0 * s], src[(c0 + 1) * s], src[(c0 + 2) * s]};
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // cells c-2..c+2
     double lvm = c0 >= 1 ? fr[(c0 - 1) * s] : 0.0;
     double lvp = c0 <= nd ? fl[c0 * s] : 0.0;
-    for (int c = c0; c < c1; ++c) {
-        const double xn = c + 3 <= nd + 3 ? src[(c + 3) * s] : 0.0;
-        const double lvm_n = fr[c * s];  // face c seeds vm_out of cell c+1
-        const double lvp_n = c + 1 <= nd ? fl[(c + 1) * s] : 0.0;
-        recon_adj<RECON>(A, c, x, lvm, lvp, acc);
-        emit(c - 2, acc[0]);
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            acc[m] = acc[m + 1];
-            x[m] = x[m + 1];
+    if constexpr (RECON == 4) {
+        const double xa = src[(c0 - 2) * s], xb = src[(c0 - 1) * s];
+        double x0 = src[c0 * s], x1 = src[(c0 + 1) * s], x2 = src[(c0 + 2) * s];  // cells c, c+1, c+2
+        PpmSlope sm = ppm_slope_grad(xa, xb, x0, A.s0[c0 - 1], A.s1[c0 - 1]);      // of cell c-1
+        PpmSlope sc = ppm_slope_grad(xb, x0, x1, A.s0[c0], A.s1[c0]);              // of cell c
+        double V = ppm_face(xb, x0, sm.d, sc.d, A.a0[c0 - 1], A.a1[c0 - 1], A.a2[c0 - 1], A.a3[c0 - 1]);
+        double lr = 0.0, ld = 0.0;                // vr adjoint of cell c-1; slope adjoint of cell c-1
+        double am = 0.0, ab = 0.0, ac = 0.0;      // value adjoints of cells c-2, c-1, c
+        // the face between cells c-1 and c with adjoint L, then the slope of cell c-1
+        auto close = [&](int c, double L, double& ld_c) {
+            const double sL = (A.a0[c - 1] + A.a1[c - 1]) * L;
+            ab += L - sL;
+            ac += sL;
+            const double l1 = ld + A.a3[c - 1] * L;
+            ld_c = A.a2[c - 1] * L;
+            am += l1 * sm.gm;
+            ab -= l1 * (sm.gm + sm.gp);
+            ac += l1 * sm.gp;
+        };
+        for (int c = c0; c < c1; ++c) {
+            const double xn = c + 3 <= nd + 3 ? src[(c + 3) * s] : 0.0;
+            const double lvm_n = fr[c * s];  // face c seeds vm_out of cell c+1
+            const double lvp_n = c + 1 <= nd ? fl[(c + 1) * s] : 0.0;
+            const PpmSlope sp = ppm_slope_grad(x0, x1, x2, A.s0[c + 1], A.s1[c + 1]);
+            const double Vr = ppm_face(x0, x1, sc.d, sp.d, A.a0[c], A.a1[c], A.a2[c], A.a3[c]);
+            const PpmFixAdj f = ppm_fix_adj(x0, V, Vr, lvm, lvp);
+            double ld_c;
+            close(c, lr + f.l, ld_c);
+            ac += f.c;
+            emit(c - 2, am);
+            am = ab;
+            ab = ac;
+            ac = 0.0;
+            lr = f.r;
+            ld = ld_c;
+            sm = sc;
+            sc = sp;
+            V = Vr;
+            x0 = x1;
+            x1 = x2;
+            x2 = xn;
+            lvm = lvm_n;
+            lvp = lvp_n;
         }
-        acc[4] = 0.0;
-        x[4] = xn;
-        lvm = lvm_n;
-        lvp = lvp_n;
-    }
+        // the last face (c1-1 | c1), and the slopes of cells c1-1 and c1
+        double ld_c;
+        close(c1, lr, ld_c);
+        emit(c1 - 2, am);
+        emit(c1 - 1, ab + ld_c * sc.gm);
+        emit(c1, ac - ld_c * (sc.gm + sc.gp));
+        emit(c1 + 1, ld_c * sc.gp);
+    } else {
+        double x[5] = {src[(c0 - 2) * s], src[(c0 - 1) * s], src[c0 * s], src[(c0 + 1) * s], src[(c0 + 2) * s]};
+        double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // cells c-2..c+2
+        for (int c = c0; c < c1; ++c) {
+            const double xn = c + 3 <= nd + 3 ? src[(c + 3) * s] : 0.0;
+            const double lvm_n = fr[c * s];
+            const double lvp_n = c + 1 <= nd ? fl[(c + 1) * s] : 0.0;
+            tvd_adj(A, c, x, lvm, lvp, acc);
+            emit(c - 2, acc[0]);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) emit(c1 - 2 + m, acc[m]);
+            for (int m = 0; m < 4; ++m) {
+                acc[m] = acc[m + 1];
+                x[m] = x[m + 1];
+            }
+            acc[4] = 0.0;
+            x[4] = xn;
+            lvm = lvm_n;
+            lvp = lvp_n;
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) emit(c1 - 2 + m, acc[m]);
+    }
 }
 
 // sweep^T, pass B along x: the reconstruction transpose with one lane per
-// cell. A warp covers cells 28w-4 .. 28w+27 of a row and owns the middle 28
-// (lanes 2..29): each lane transposes its own cell's reconstruction, and the
-// five contributions to each owned cell are summed through warp shuffles.
+// cell, one warp per (row, field, RX_CELLS cells). A warp covers 32 cells of a
+// row and owns its middle RX_CELLS: each lane forms its own cell's slope,
+// interface value and fix, and the neighbours' shares come through shuffles (a
+// cell's adjoint reaches four cells to either side).
+constexpr int RX_CELLS = 24;
+inline long long recon_x_warps(const Box& b) {
+    return (long long)(b.ny + 2) * (b.nz + 2) * ((b.nx + 6 + RX_CELLS - 1) / RX_CELLS);
+}
 template <int RECON>
 __global__ void __launch_bounds__(128) k_adj_recon_x(Box b, Tabs T, Prim pr, FaceAdj fa, AdjPrim o) {
-    const int nw = (b.nx + 6 + 27) / 28;  // warps per row
+    constexpr unsigned FULL = 0xffffffffu;
+    const int nw = (b.nx + 6 + RX_CELLS - 1) / RX_CELLS;  // warps per row
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const long long rows = (long long)(b.ny + 2) * (b.nz + 2);
@@ -732,28 +784,39 @@ __global__ void __launch_bounds__(128) k_adj_recon_x(Box b, Tabs T, Prim pr, Fac
     const int w = (int)(warp % nw);
     const long long row = warp / nw;
     const int k = (int)(row % (b.ny + 2)), l = (int)(row / (b.ny + 2));
-    const int c = 28 * w + lane - 4;
+    const int c = RX_CELLS * w + lane - 6;  // owned: lanes 4..27, from cell -2
     const AxisTabs A = T.ax[0];
-    const int base = b.idx(0, k, l);
-    const bool mine = c >= 0 && c <= b.nx + 1;                  // a reconstructed cell
-    const bool owned = lane >= 2 && lane <= 29 && c >= -2 && c <= b.nx + 3;
-#pragma unroll 1
-    for (int v = 0; v < 7; ++v) {
-        const double* src;
-        double* dst;
-        sweep_field<0>(pr, o, v, src, dst);
+    const int at = b.idx(0, k, l) + c;
+    const bool mine = c >= 0 && c <= b.nx + 1;  // a reconstructed cell
+    const bool owned = lane >= 4 && lane <= 27 && c <= b.nx + 3;
+    const int ct = min(max(c, -1), b.nx + 1);  // table index of the lane's cell and its upper face
+    const double* src;
+    double* dst;
+    sweep_field<0>(pr, o, (int)blockIdx.y, src, dst);
+    const double x = c >= -2 && c <= b.nx + 3 ? src[at] : 0.0;
+    const double lvm = mine && c >= 1 ? fa.r[blockIdx.y][at - 1] : 0.0;
+    const double lvp = mine && c <= b.nx ? fa.l[blockIdx.y][at] : 0.0;
+    const double xm = __shfl_up_sync(FULL, x, 1), xp = __shfl_down_sync(FULL, x, 1);
+    double tot;
+    if constexpr (RECON == 4) {
+        const int cs = min(max(c, -1), b.nx + 2);  // slopes exist on -1..nx+2
+        const PpmSlope s = ppm_slope_grad(xm, x, xp, A.s0[cs], A.s1[cs]);
+        const double a2 = A.a2[ct], a3 = A.a3[ct], as = A.a0[ct] + A.a1[ct];
+        const double V = ppm_face(x, xp, s.d, __shfl_down_sync(FULL, s.d, 1), A.a0[ct], A.a1[ct], a2, a3);  // c | c+1
+        const PpmFixAdj f = ppm_fix_adj(x, __shfl_up_sync(FULL, V, 1), V, lvm, lvp);
+        const double L = f.r + __shfl_down_sync(FULL, f.l, 1);  // adjoint of V
+        const double sL = as * L;
+        // value and slope adjoints: from the face above (L) and the one below
+        const double ld = a3 * L + __shfl_up_sync(FULL, a2 * L, 1);
+        tot = (f.c + (L - sL)) + __shfl_up_sync(FULL, sL, 1) - ld * (s.gm + s.gp);
+        tot += __shfl_down_sync(FULL, ld * s.gm, 1) + __shfl_up_sync(FULL, ld * s.gp, 1);
+    } else {
         double lv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        if (mine) {
-            const double* q = src + base + c;
-            const double x[5] = {q[-2], q[-1], q[0], q[1], q[2]};
-            const double lvm = c >= 1 ? fa.r[v][base + c - 1] : 0.0;
-            const double lvp = c <= b.nx ? fa.l[v][base + c] : 0.0;
-            recon_adj<RECON>(A, c, x, lvm, lvp, lv);
-        }
-        const double tot = lv[2] + __shfl_down_sync(0xffffffffu, lv[0], 2) + __shfl_down_sync(0xffffffffu, lv[1], 1) +
-                           __shfl_up_sync(0xffffffffu, lv[3], 1) + __shfl_up_sync(0xffffffffu, lv[4], 2);
-        if (owned && tot != 0.0) dst[base + c] += tot;
+        const double v[5] = {0.0, xm, x, xp, 0.0};
+        if (mine) tvd_adj(A, c, v, lvm, lvp, lv);
+        tot = lv[2] + __shfl_down_sync(FULL, lv[1], 1) + __shfl_up_sync(FULL, lv[3], 1);
     }
+    if (owned && tot != 0.0) dst[at] += tot;
 }
 
 // boundary^T: the transpose of k_boundary, in gather form. k_boundary copies
@@ -795,6 +858,9 @@ __global__ void __launch_bounds__(256) k_adj_boundary_gather(Box b, BoundArgs fw
                                                              double* lbz) {
     int j, k, l, i;
     if (!box1_index(b, j, k, l, i)) return;
+    // ghosts copy from the three cells next to a face only
+    auto inner = [](int i, int n) { return i == 0 || (i > 3 && i < n - 2); };
+    if (inner(j, b.nx) && inner(k, b.ny) && inner(l, b.nz)) return;
     // index lists per direction: entry 0 is the identity, then the ghost images
     int gx[7], sx[7], gy[7], sy[7], gz[7], sz[7], gye[7], sye[7];
     gx[0] = j, gy[0] = k, gz[0] = l, gye[0] = k;
@@ -902,6 +968,36 @@ __global__ void __launch_bounds__(256) k_adj_boundary_clear(Box b, BoundArgs fw,
     if (l >= 0 && l <= b.nz && (gx || gy)) lbz[i] = 0.0;
 }
 
+// the primitives (before the boundary fill) and face fields of a taped combine
+// output src, into a scratch state: k_utop on the tape's own arrays, without a
+// copy of them first. The scratch state's hydro cons are not read.
+template <int MODEL>
+__global__ void __launch_bounds__(256) k_adj_prims(Box b, Arr8 src, UtopArgs a) {
+    int j, k, l, i;
+    if (!box1_index(b, j, k, l, i)) return;
+    const bool interior = j >= 1 && k >= 1 && l >= 1;
+    const int off[3] = {1, b.SX, b.SX * b.SY};
+    double uh[5], bc[3];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) uh[q] = src.a[q][i];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double f = src.a[IBX + q][i];
+        a.u[IBX + q][i] = f;
+        bc[q] = interior ? 0.5 * (f + src.a[IBX + q][i - off[q]]) : a.bc[q][i];
+        if (interior) a.bc[q][i] = bc[q];
+    }
+    const CellConv o =
+        utop_of<MODEL, true, true>(uh, interior, bc[0], bc[1], bc[2], a.ggas, a.rho_floor, a.eps_floor);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a.w[q][i] = o.w[q];
+    a.eps[i] = o.eps;
+    if (interior) {
+        a.w[4][i] = o.p;
+        if (o.bad) atomicOr(a.flag, 1u);
+    }
+}
+
 // utop^T on the active cells: from the adjoints of the re-derived conserved
 // hydro variables (lu) and of the primitives (o), the adjoint of the
 // combine's output Upre (hydro part, mu) and of the cell-centred field
@@ -934,14 +1030,18 @@ __global__ void __launch_bounds__(256) k_adj_utop(Box b, Arr8 u, Arr8 w0, const 
     const double by = 0.5 * (u.a[IBY][i] + u.a[IBY][i - b.SX]);
     const double bz = 0.5 * (u.a[IBZ][i] + u.a[IBZ][i - b.SX * b.SY]);
     const double bsquare = (bx * bx + by * by) + bz * bz;
-    double rho, vx, vy, vz, e_raw;
+    double rho, vx, vy, vz, e_raw, ir = 0.0, eb = 0.0;  // ir = 1/rho, eb = (E - bsq/2)/rho
     if (FROM_CONS) {
         rho = u.a[IRHO][i];
-        vx = u.a[IVX][i] / rho;
-        vy = u.a[IVY][i] / rho;
-        vz = u.a[IVZ][i] / rho;
-        const double vsq = (vx * vx + vy * vy) + vz * vz;
-        e_raw = (u.a[ITAU][i] - 0.5 * bsquare) / rho - 0.5 * vsq;
+        ir = 1.0 / rho;
+        const double n[4] = {u.a[IVX][i], u.a[IVY][i], u.a[IVZ][i], u.a[ITAU][i] - 0.5 * bsquare};
+        double q[4];
+        quot_group(n, rho, q);  // the forward's values: e_raw decides a branch
+        vx = q[0];
+        vy = q[1];
+        vz = q[2];
+        eb = q[3];
+        e_raw = eb - 0.5 * ((vx * vx + vy * vy) + vz * vz);
     } else {
         rho = w0.a[0][i];
         vx = w0.a[1][i];
@@ -964,19 +1064,18 @@ __global__ void __launch_bounds__(256) k_adj_utop(Box b, Arr8 u, Arr8 w0, const 
     if (clamped) Le = 0.0;
     if (FROM_CONS) {
         // e_raw = (E - bsq/2)/rho - vsq/2
-        const double E = u.a[ITAU][i];
-        const double LE = Le / rho;
-        Lbsq -= 0.5 * Le / rho;
-        Lrho -= Le * (E - 0.5 * bsquare) / (rho * rho);
+        const double LE = Le * ir;
+        Lbsq -= 0.5 * LE;
+        Lrho -= LE * eb;
         Lvsq -= 0.5 * Le;
         Lvx += 2.0 * vx * Lvsq;
         Lvy += 2.0 * vy * Lvsq;
         Lvz += 2.0 * vz * Lvsq;
         // v = m / rho
-        mu.a[IVX][i] = Lvx / rho;
-        mu.a[IVY][i] = Lvy / rho;
-        mu.a[IVZ][i] = Lvz / rho;
-        Lrho -= (Lvx * vx + Lvy * vy + Lvz * vz) / rho;
+        mu.a[IVX][i] = Lvx * ir;
+        mu.a[IVY][i] = Lvy * ir;
+        mu.a[IVZ][i] = Lvz * ir;
+        Lrho -= (Lvx * vx + Lvy * vy + Lvz * vz) * ir;
         mu.a[IRHO][i] = Lrho;
         mu.a[ITAU][i] = LE;
     } else {

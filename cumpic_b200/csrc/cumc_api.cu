@@ -75,6 +75,9 @@ struct cumc_ctx {
     double prof_ms[CUMC_K_COUNT]{};
     long long launches = 0;
 
+    cudaGraphExec_t rk_exec = nullptr;  // the launches of one cumc_rungekutta (rk_step_host)
+    long long rk_launches = 0;
+    int rk_calls = 0;
     cudaGraphExec_t graph_exec = nullptr;
     double graph_t_end = 0.0;
     long long graph_launches_per_step = 0;
@@ -760,6 +763,43 @@ void rk_step(cumc_ctx* c, const Box& b) {
     run_stage(c, b, 3);
 }
 
+// The step of cumc_rungekutta. Its launches are the same every call (dt and the
+// state stay in their places on the device), so from the second call on they
+// go as one graph: on small boxes the host's launches took longer than the
+// kernels. Launched one by one under per-kernel timing and while the caller
+// captures the stream.
+int rk_step_host(cumc_ctx* c) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUMC_CHECK(cudaStreamIsCapturing(c->stream, &cap));
+    const bool plain = c->prof_on || cap != cudaStreamCaptureStatusNone || (!c->rk_exec && c->rk_calls++ == 0);
+    if (!plain && !c->rk_exec) {
+        cudaGraph_t g;
+        const long long before = c->launches;
+        CUMC_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        c->fuse_dt = true;
+        rk_step(c, c->box);
+        c->fuse_dt = false;
+        c->rk_launches = c->launches - before;
+        c->launches = before;
+        CUMC_CHECK(cudaStreamEndCapture(c->stream, &g));
+        const cudaError_t e = cudaGraphInstantiate(&c->rk_exec, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) {
+            c->rk_exec = nullptr;
+            return cuda_fail(c, e, "cudaGraphInstantiate");
+        }
+    }
+    if (plain) {
+        c->fuse_dt = true;
+        rk_step(c, c->box);
+        c->fuse_dt = false;
+    } else {
+        CUMC_CHECK(cudaGraphLaunch(c->rk_exec, c->stream));
+        c->launches += c->rk_launches;
+    }
+    return CUMC_OK;
+}
+
 void finddt_launch(cumc_ctx* c, const Box& b) {
     launch(c, -1, 1, 1, k_reset_dtmin, c->dtmin);
     if (c->mixed) {
@@ -793,10 +833,8 @@ Clock make_clock(cumc_ctx* c) {
 void loop_step(cumc_ctx* c, double t_end) {
     Box b = c->box;
     const Clock k = make_clock(c);
-    launch(c, -1, 1, 1, k_check_done, k, t_end);
+    launch(c, -1, 1, 1, k_step_begin, k, t_end);
     b.skip = k.done;
-    launch(c, -1, 1, 1, k_clip_dt, k, t_end);
-    launch(c, -1, 1, 1, k_reset_dtmin, c->dtmin);
     c->fuse_dt = true;
     rk_step(c, b);
     c->fuse_dt = false;
@@ -1229,6 +1267,7 @@ int cumc_free(cumc_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (auto& pe : c->prof) { cudaEventDestroy(pe.a); cudaEventDestroy(pe.b); }
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
+    if (c->rk_exec) cudaGraphExecDestroy(c->rk_exec);
     for (void* p : c->allocs) cudaFree(p);
     if (c->adj_slab) cudaFree(c->adj_slab);
     if (c->snap_stream) {
@@ -1374,13 +1413,10 @@ int cumc_rungekutta(cumc_ctx* c, double dt) {
     if (c->exchange) return c->fail(CUMC_ERR_STATE, "a slab with CUMC_BC_EXCHANGE faces steps by cumc_rk_stage and the halo exchange");
     if (c->next_stage != 1) return c->fail(CUMC_ERR_STATE, "cumc_rk_stage left a step unfinished");
     if (!(dt >= 0.0 && std::isfinite(dt))) return c->fail(CUMC_ERR_ARG, "dt must be finite and non-negative");
-    launch(c, -1, 1, 1, k_set_scalar, c->scal, dt);
     // stage 3 forms the next step's CFL dt, which cumc_finddt then returns
     // without a pass over the state (the same expression, so the same bits)
-    launch(c, -1, 1, 1, k_reset_dtmin, c->dtmin);
-    c->fuse_dt = true;
-    rk_step(c, c->box);
-    c->fuse_dt = false;
+    launch(c, -1, 1, 1, k_set_dt, make_clock(c), dt);
+    if ((rc = rk_step_host(c)) != CUMC_OK) return rc;
     c->dt_valid = true;
     return sync_status(c);
 }
@@ -1678,14 +1714,6 @@ void copy_state(cumc_ctx* c, StateSet dst, StateSet src) {
         cudaMemcpyAsync(*dst.all(i), *src.all(i), bytes, cudaMemcpyDeviceToDevice, c->stream);
 }
 
-// primitives (and boundary-filled face fields) of a taped combine output
-void adj_prims_from(cumc_ctx* c, const Box& b, double* const* upre, StateSet& P) {
-    const size_t bytes = (size_t)b.count() * sizeof(double);
-    for (int q = 0; q < 8; ++q) cudaMemcpyAsync(P.u[q], upre[q], bytes, cudaMemcpyDeviceToDevice, c->stream);
-    utop_into(c, b, P.u, P.prim(), true);
-    boundary_into(c, b, P.u, P.prim());
-}
-
 Arr8 arr8(double* const* p, int n = 8) {
     Arr8 a{};
     for (int q = 0; q < n; ++q) a.a[q] = p[q];
@@ -1695,6 +1723,15 @@ Arr3 arr3(double* const* p) {
     Arr3 a;
     for (int q = 0; q < 3; ++q) a.a[q] = p[q];
     return a;
+}
+
+// primitives (and boundary-filled face fields) of a taped combine output
+void adj_prims_from(cumc_ctx* c, const Box& b, double* const* upre, StateSet& P) {
+    const long long n = (long long)(b.nx + 1) * (b.ny + 1) * (b.nz + 1);
+    const UtopArgs a = utop_args(c, P.u, P.prim());
+    if (c->model == CUMC_MODEL_RIEMANN) launch(c, CUMC_K_UTOP, n, 256, k_adj_prims<1>, b, arr8(upre), a);
+    else launch(c, CUMC_K_UTOP, n, 256, k_adj_prims<0>, b, arr8(upre), a);
+    boundary_into(c, b, P.u, P.prim());
 }
 
 // reconstruction transpose along y or z: the even segments, then the odd
@@ -1730,11 +1767,11 @@ void adj_sweeps(cumc_ctx* c, const Box& b, const Prim& pr, const AdjStage& st, c
         launch_grid(c, -1, grid, WK_THREADS, walk_smem<double>(D), k_sweep_walk_sm<D, RECON, double, true>, b, c->tabs,
                     pr, c->ggas, sl, seg, sr, 0, -1);
     };
-    // x: pass A per face, pass B one lane per cell (28 owned cells a warp)
+    // x: pass A per face, pass B one lane per cell and field
     launch(c, -1, xwarp_threads(b), 128, k_sweep_xwarp<RECON, double, true>, b, c->tabs, pr, c->ggas, sl, sr, 0, -1);
     launch(c, -1, fx, 128, k_adj_hll<COORD, 0, RECON, true>, b, c->tabs, pr, c->ggas, st, fa, lbf[0]);
-    const long long xwarps = (long long)(b.ny + 2) * (b.nz + 2) * ((b.nx + 6 + 27) / 28);
-    launch(c, -1, xwarps * 32, 128, k_adj_recon_x<RECON>, b, c->tabs, pr, fa, lp);
+    launch_grid(c, -1, dim3((unsigned)((recon_x_warps(b) * 32 + 127) / 128), 7), 128, 0, k_adj_recon_x<RECON>, b,
+                c->tabs, pr, fa, lp);
     // y, z: pass A per face, pass B one thread per (column, field)
     states(std::integral_constant<int, 1>{});
     launch(c, -1, fy, 128, k_adj_hll<COORD, 1, RECON, true>, b, c->tabs, pr, c->ggas, st, fa, lbf[1]);

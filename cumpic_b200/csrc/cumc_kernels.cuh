@@ -962,15 +962,23 @@ struct Clock {
 
 static __global__ void k_set_scalar(double* p, double v) { *p = v; }
 static __global__ void k_reset_dtmin(unsigned long long* p) { *p = (unsigned long long)__double_as_longlong(1.0e10); }
-// loop condition of solver/main.f90:127
-static __global__ void k_check_done(Clock c, double t_end) { *c.done = (*c.t < t_end) ? 0 : 1; }
-// dt = finddt, clipped to t_end (solver/main.f90:133-135)
-static __global__ void k_clip_dt(Clock c, double t_end) {
-    if (*c.done) return;
-    double dt = __longlong_as_double((long long)*c.dtmin);
-    const double t = *c.t;
-    if (t + dt > t_end) dt = t_end - t;
+// dt of a host-driven step, and dtmin cleared for the next one's
+static __global__ void k_set_dt(Clock c, double dt) {
     *c.dt = dt;
+    *c.dtmin = (unsigned long long)__double_as_longlong(1.0e10);
+}
+// start of a device-driven step: the loop condition of solver/main.f90:127,
+// dt = finddt clipped to t_end (solver/main.f90:133-135), dtmin cleared for the
+// next step's
+static __global__ void k_step_begin(Clock c, double t_end) {
+    const double t = *c.t;
+    const bool done = !(t < t_end);
+    *c.done = done ? 1 : 0;
+    if (!done) {
+        const double dt = __longlong_as_double((long long)*c.dtmin);
+        *c.dt = t + dt > t_end ? t_end - t : dt;
+    }
+    *c.dtmin = (unsigned long long)__double_as_longlong(1.0e10);
 }
 static __global__ void k_advance_time(Clock c) {
     if (*c.done) return;
