@@ -337,9 +337,9 @@ template <int COORD>
 __global__ void __launch_bounds__(256) k_adj_ct(Box b, Tabs T, AdjStage a, double* lex, double* ley, double* lez) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / ((long long)n0 * n1));
+    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     const int sj = 1, sk = b.SX, sl = b.SX * b.SY;
     const double cdt = a.gam * *a.dt;
@@ -379,9 +379,9 @@ __global__ void __launch_bounds__(256) k_adj_ecell(Box b, Prim pr, const double*
                                                    const double* lez, AdjPrim o) {
     const int n0 = b.nx + 2, n1 = b.ny + 2, n2 = b.nz + 2;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / ((long long)n0 * n1));
+    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     const int sj = 1, sk = b.SX, sl = b.SX * b.SY;
     auto E = [&](const double* e, int dj, int dk, int dl) -> double {
@@ -410,9 +410,9 @@ __global__ void __launch_bounds__(256) k_adj_ecell(Box b, Prim pr, const double*
 template <int COORD>
 __global__ void __launch_bounds__(256) k_adj_source(Box b, Tabs T, Prim pr, AdjStage a, int repeat, AdjPrim o) {
     const long long total = (long long)b.nx * b.ny * b.nz;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    const int j = (int)(t % b.nx) + 1, k = (int)((t / b.nx) % b.ny) + 1, l = (int)(t / ((long long)b.nx * b.ny)) + 1;
+    const int j = (int)(t % b.nx) + 1, k = (int)((t / b.nx) % b.ny) + 1, l = (int)(t / b.nx / b.ny) + 1;
     const int i = b.idx(j, k, l);
     const double f = (a.gam * *a.dt) * repeat;
     const double lx = f * a.mu[IVX][i], ly = f * a.mu[IVY][i], lz = f * a.mu[IVZ][i];
@@ -481,9 +481,9 @@ __global__ void __launch_bounds__(128, CUMC_ADJ_MINB) k_adj_hll(Box b, Tabs T, P
     const int n1 = (DIR == 1 ? b.ny : b.ny + 1) + 1;
     const int n2 = (DIR == 2 ? b.nz : b.nz + 1) + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / ((long long)n0 * n1));
+    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / n0 / n1);
     const int base = b.idx(j, k, l);
     const int sj = 1, sk = b.SX, sl = b.SX * b.SY;
     const int s = DIR == 0 ? sj : DIR == 1 ? sk : sl;
@@ -595,7 +595,10 @@ __global__ void __launch_bounds__(128, CUMC_ADJ_MINB) k_adj_hll(Box b, Tabs T, P
     lambf[base] += lbn;
 }
 
-// field v (0..6) of a sweep along DIR: source and adjoint arrays
+// field v (0..6) of a sweep along DIR: source and adjoint arrays. (v is not a
+// constant here: the kernels below take their arrays as grid constants, which
+// are indexed in place. As plain parameters they were copied to 272 bytes of
+// stack by every thread first: k_adj_recon_x 795 us a launch at 128^3.)
 template <int DIR>
 __device__ __forceinline__ void sweep_field(const Prim& pr, const AdjPrim& o, int v, const double*& src, double*& dst) {
     constexpr int bt_a = DIR == 0 ? 1 : 0;
@@ -664,9 +667,11 @@ __device__ __forceinline__ PpmFixAdj ppm_fix_adj(double vc, double vl, double vr
 constexpr int RC_SEG = 32;
 
 template <int DIR, int RECON>
-__global__ void __launch_bounds__(128) k_adj_recon_col(Box b, Tabs T, Prim pr, FaceAdj fa, AdjPrim o, int parity) {
+__global__ void __launch_bounds__(128) k_adj_recon_col(Box b, const __grid_constant__ Tabs T, const __grid_constant__ Prim pr,
+                                                       const __grid_constant__ FaceAdj fa,
+                                                       const __grid_constant__ AdjPrim o, int parity) {
     using G = WalkGeom<DIR>;
-    const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= G::ncols(b)) return;
     const int v = blockIdx.y;
     const int nd = G::nd(b);
@@ -774,16 +779,17 @@ inline long long recon_x_warps(const Box& b) {
     return (long long)(b.ny + 2) * (b.nz + 2) * ((b.nx + 6 + RX_CELLS - 1) / RX_CELLS);
 }
 template <int RECON>
-__global__ void __launch_bounds__(128) k_adj_recon_x(Box b, Tabs T, Prim pr, FaceAdj fa, AdjPrim o) {
+__global__ void __launch_bounds__(128) k_adj_recon_x(Box b, const __grid_constant__ Tabs T, const __grid_constant__ Prim pr,
+                                                     const __grid_constant__ FaceAdj fa,
+                                                     const __grid_constant__ AdjPrim o) {
     constexpr unsigned FULL = 0xffffffffu;
     const int nw = (b.nx + 6 + RX_CELLS - 1) / RX_CELLS;  // warps per row
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // 32-bit index arithmetic (fewer warps than cells, fewer than 2^31 cells)
+    const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    const long long rows = (long long)(b.ny + 2) * (b.nz + 2);
-    if (warp >= rows * nw) return;  // whole warp
-    const int w = (int)(warp % nw);
-    const long long row = warp / nw;
-    const int k = (int)(row % (b.ny + 2)), l = (int)(row / (b.ny + 2));
+    const unsigned row = warp / nw;
+    const int w = (int)(warp - row * nw), k = (int)(row % (b.ny + 2)), l = (int)(row / (b.ny + 2));
+    if (l > b.nz + 1) return;  // whole warp
     const int c = RX_CELLS * w + lane - 6;  // owned: lanes 4..27, from cell -2
     const AxisTabs A = T.ax[0];
     const int at = b.idx(0, k, l) + c;
@@ -854,13 +860,45 @@ __device__ __forceinline__ int bsign(const BoundArgs& fw, int dir, int side, int
     return fw.fac[2 * dir + side][q];
 }
 
-__global__ void __launch_bounds__(256) k_adj_boundary_gather(Box b, BoundArgs fw, AdjPrim o, double* lbx, double* lby,
-                                                             double* lbz) {
-    int j, k, l, i;
-    if (!box1_index(b, j, k, l, i)) return;
-    // ghosts copy from the three cells next to a face only
-    auto inner = [](int i, int n) { return i == 0 || (i > 3 && i < n - 2); };
-    if (inner(j, b.nx) && inner(k, b.ny) && inner(l, b.nz)) return;
+// A ghost's source lies within three cells of a face, so only cells with an
+// index in the face set 0..3, n-2..n of some direction are visited: one thread
+// a box cell spent 119 us at 128^3, half its warps on the few such cells of
+// every row.
+__host__ __device__ __forceinline__ int face_set(int n) { return n + 1 < 7 ? n + 1 : 7; }  // its size
+__device__ __forceinline__ int face_set_index(int s, int n) { return n + 1 < 7 || s < 4 ? s : n - 6 + s; }
+inline long long face_set_cells(const Box& b) {
+    const long long n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
+    const long long i0 = n0 - face_set(b.nx), i1 = n1 - face_set(b.ny), i2 = n2 - face_set(b.nz);
+    return n0 * n1 * n2 - i0 * i1 * i2;
+}
+
+__global__ void __launch_bounds__(256) k_adj_boundary_gather(Box b, const __grid_constant__ BoundArgs fw,
+                                                             const __grid_constant__ AdjPrim o, double* lbx,
+                                                             double* lby, double* lbz) {
+    // the planes l in the face set, then the rows k in it of the other planes,
+    // then the cells j in it of the other rows (the seven of a row on
+    // consecutive threads)
+    const int n0 = b.nx + 1, n1 = b.ny + 1, fx = face_set(b.nx), fy = face_set(b.ny), fz = face_set(b.nz);
+    const unsigned nz = (unsigned)fz * n0 * n1, ny = (unsigned)(b.nz + 1 - fz) * fy * n0;
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    int j, k, l;
+    if (t < nz) {
+        j = (int)(t % n0);
+        k = (int)((t / n0) % n1);
+        l = face_set_index((int)(t / n0 / n1), b.nz);
+    } else if ((t -= nz) < ny) {
+        j = (int)(t % n0);
+        k = face_set_index((int)((t / n0) % fy), b.ny);
+        l = 4 + (int)(t / n0 / fy);
+    } else {
+        t -= ny;
+        const unsigned rows = (unsigned)(n1 - fy) * (b.nz + 1 - fz);
+        if (t >= rows * fx) return;
+        j = face_set_index((int)(t % fx), b.nx);
+        k = 4 + (int)((t / fx) % (n1 - fy));
+        l = 4 + (int)(t / fx / (n1 - fy));
+    }
+    const int i = b.idx(j, k, l);
     // index lists per direction: entry 0 is the identity, then the ghost images
     int gx[7], sx[7], gy[7], sy[7], gz[7], sz[7], gye[7], sye[7];
     gx[0] = j, gy[0] = k, gz[0] = l, gye[0] = k;
@@ -932,24 +970,21 @@ __global__ void __launch_bounds__(256) k_adj_boundary_gather(Box b, BoundArgs fw
 // the ghost order of k_boundary)
 __global__ void __launch_bounds__(256) k_adj_boundary_clear(Box b, BoundArgs fw, AdjPrim o, double* lbx, double* lby,
                                                             double* lbz) {
-    const long long zsl = 6LL * b.SX * b.SY, ysl = 6LL * b.SX * b.nz, xsl = 6LL * b.ny * b.nz;
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned zp = (unsigned)b.SX * b.SY, yp = (unsigned)b.SX * b.nz, xp = (unsigned)b.ny * b.nz;
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     int j, k, l;
-    if (t < zsl) {
-        const int s = (int)(t / ((long long)b.SX * b.SY));
-        const int r = (int)(t % ((long long)b.SX * b.SY));
+    if (t < 6u * zp) {
+        const int s = (int)(t / zp), r = (int)(t % zp);
         l = s < 3 ? s - 2 : b.nz + s - 2;
         k = r / b.SX - 2;
         j = r % b.SX - 2;
-    } else if ((t -= zsl) < ysl) {
-        const int s = (int)(t / ((long long)b.SX * b.nz));
-        const int r = (int)(t % ((long long)b.SX * b.nz));
+    } else if ((t -= 6u * zp) < 6u * yp) {
+        const int s = (int)(t / yp), r = (int)(t % yp);
         k = s < 3 ? s - 2 : b.ny + s - 2;
         l = r / b.SX + 1;
         j = r % b.SX - 2;
-    } else if ((t -= ysl) < xsl) {
-        const int s = (int)(t / ((long long)b.ny * b.nz));
-        const int r = (int)(t % ((long long)b.ny * b.nz));
+    } else if ((t -= 6u * yp) < 6u * xp) {
+        const int s = (int)(t / xp), r = (int)(t % xp);
         j = s < 3 ? s - 2 : b.nx + s - 2;
         l = r / b.ny + 1;
         k = r % b.ny + 1;
@@ -1012,9 +1047,9 @@ __global__ void __launch_bounds__(256) k_adj_utop(Box b, Arr8 u, Arr8 w0, const 
                                                   double beta, Arr8 lam0) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / ((long long)n0 * n1));
+    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     if (!(j >= 1 && k >= 1 && l >= 1)) {
 #pragma unroll
@@ -1110,9 +1145,9 @@ __global__ void __launch_bounds__(256) k_adj_bface(Box b, Arr3 lbf, Arr3 lb, Arr
                                                    Arr3 lam0) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
-    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / ((long long)n0 * n1));
+    const int j = (int)(t % n0), k = (int)((t / n0) % n1), l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     const int st[3] = {1, b.SX, b.SX * b.SY};
     const int own[3] = {j, k, l};
@@ -1145,10 +1180,10 @@ __global__ void __launch_bounds__(256) k_adj_bface(Box b, Arr3 lbf, Arr3 lb, Arr
 __global__ void __launch_bounds__(256) k_adj_objective(Box b, Tabs T, int coord, Prim pr, Arr8 u, int kind, AdjPrim o,
                                                        Arr8 lamu, double* partial) {
     const long long total = (long long)b.nx * b.ny * b.nz;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     double acc = 0.0;
     if (t < total) {
-        const int j = (int)(t % b.nx) + 1, k = (int)((t / b.nx) % b.ny) + 1, l = (int)(t / ((long long)b.nx * b.ny)) + 1;
+        const int j = (int)(t % b.nx) + 1, k = (int)((t / b.nx) % b.ny) + 1, l = (int)(t / b.nx / b.ny) + 1;
         const int i = b.idx(j, k, l);
         // cell volume: dx dy dz; R dR dphi dz; (r^3)/3 d(-cos theta) dphi
         const double dv = coord == CUMC_CARTESIAN     ? (T.ax[0].d[j] * T.ax[1].d[k]) * T.ax[2].d[l]
@@ -1193,9 +1228,9 @@ __global__ void __launch_bounds__(256) k_adj_objective(Box b, Tabs T, int coord,
 
 // clears the weights of a linear objective off its live entries
 __global__ void __launch_bounds__(256) k_adj_mask_live(Box b, Arr8 lamu) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= b.count()) return;
-    const int j = (int)(t % b.SX) - 2, k = (int)((t / b.SX) % b.SY) - 2, l = (int)(t / ((long long)b.SX * b.SY)) - 2;
+    const int j = (int)(t % b.SX) - 2, k = (int)((t / b.SX) % b.SY) - 2, l = (int)(t / b.SX / b.SY) - 2;
     const int own[3] = {j, k, l};
     const int nn[3] = {b.nx, b.ny, b.nz};
     const bool cell = inside(j, k, l, b);

@@ -241,12 +241,13 @@ void launch_grid(cumc_ctx* c, int cls, dim3 grid, int block, size_t smem, K kern
     }
 }
 
-// the default x sweep of the planes l_lo .. l_lo + l_cnt - 1; pairs move as
+// the default x sweep of the l_cnt planes l_lo, l_lo + l_step, ..; pairs move as
 // vectors with an even row stride
-void sweep_xpair(cumc_ctx* c, const Box& b, const Prim& pr, const FaceFlux& out, int l_lo, int l_cnt) {
+void sweep_xpair(cumc_ctx* c, const Box& b, const Prim& pr, const FaceFlux& out, int l_lo, int l_cnt, int l_step) {
     const bool vec = xpair_vec(b, pr, out), ppm = c->recon == CUMC_PPMC;
     auto go = [&](auto kern) {
-        launch_grid(c, CUMC_K_SWEEP_X, xpair_grid(b, l_cnt), XP_THREADS, 0, kern, b, c->tabs, pr, c->ggas, out, l_lo);
+        launch_grid(c, CUMC_K_SWEEP_X, xpair_grid(b, l_cnt), XP_THREADS, 0, kern, b, c->tabs, pr, c->ggas, out, l_lo,
+                    l_step);
     };
     if (c->fast)
         vec ? go(ppm ? k_sweep_xpair<4, double, true, true> : k_sweep_xpair<1, double, true, true>)
@@ -256,10 +257,10 @@ void sweep_xpair(cumc_ctx* c, const Box& b, const Prim& pr, const FaceFlux& out,
             : go(ppm ? k_sweep_xpair<4, double, false, false> : k_sweep_xpair<1, double, false, false>);
 }
 
-// l_lo, l_cnt: the z planes whose x rows (DIR 0) or y columns (DIR 1) the
+// l_lo, l_cnt, l_step: the z planes whose x rows (DIR 0) or y columns (DIR 1) the
 // default kernels sweep (l_cnt < 0: all); the other forms sweep everything
 template <int DIR>
-void sweep(cumc_ctx* c, const Box& b, const Prim& pr, int l_lo = 0, int l_cnt = -1) {
+void sweep(cumc_ctx* c, const Box& b, const Prim& pr, int l_lo = 0, int l_cnt = -1, int l_step = 1) {
     FaceFlux out;
     for (int q = 0; q < 7; ++q) out.f[q] = c->F[DIR][q];
     // default: one lane per cell along x, the shared-memory-window walker
@@ -277,16 +278,16 @@ void sweep(cumc_ctx* c, const Box& b, const Prim& pr, int l_lo = 0, int l_cnt = 
                         (unsigned)nseg);
         const int cls = CUMC_K_SWEEP_X + DIR;
         if (mode == 4 || mode == 0 || mode == 7) {
-            const size_t sm = walk_smem<double>(DIR);
             const bool ppm = c->recon == CUMC_PPMC;
+            const size_t sm = walk_smem<double>(DIR, ppm);
             if (c->fast)
                 launch_grid(c, cls, grid, WK_THREADS, sm,
                             ppm ? k_sweep_walk_sm<DIR, 4, double, false, true> : k_sweep_walk_sm<DIR, 1, double, false, true>,
-                            b, c->tabs, pr, c->ggas, out, seg, out, c_lo, c_cnt);
+                            b, c->tabs, pr, c->ggas, out, seg, out, c_lo, c_cnt, l_step);
             else
                 launch_grid(c, cls, grid, WK_THREADS, sm,
                             ppm ? k_sweep_walk_sm<DIR, 4, double> : k_sweep_walk_sm<DIR, 1, double>, b, c->tabs, pr,
-                            c->ggas, out, seg, out, c_lo, c_cnt);
+                            c->ggas, out, seg, out, c_lo, c_cnt, l_step);
         } else {
             const size_t sm = DIR == 0 ? xstage_smem<double>() : 0;
             if (c->recon == CUMC_PPMC)
@@ -297,7 +298,7 @@ void sweep(cumc_ctx* c, const Box& b, const Prim& pr, int l_lo = 0, int l_cnt = 
         return;
     }
     if (DIR == 0 && mode == 0) {  // x: two cells a lane
-        sweep_xpair(c, b, pr, out, l_cnt >= 0 ? l_lo : 0, l_cnt >= 0 ? l_cnt : b.nz + 2);
+        sweep_xpair(c, b, pr, out, l_cnt >= 0 ? l_lo : 0, l_cnt >= 0 ? l_cnt : b.nz + 2, l_step);
         return;
     }
     if (DIR == 0 && mode == 6) {  // x: one lane per cell
@@ -336,13 +337,6 @@ int sweep_attributes(cumc_ctx* c) {
     for (const void* f : k) {
         cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw_smem<double>());
         if (e != cudaSuccess) return cuda_fail(c, e, "cudaFuncSetAttribute(sweep smem)");
-    }
-    const void* m[9] = {(const void*)k_emf_ct<1, 1>, (const void*)k_emf_ct<1, 2>, (const void*)k_emf_ct<1, 3>,
-                        (const void*)k_emf_ct<2, 1>, (const void*)k_emf_ct<2, 2>, (const void*)k_emf_ct<2, 3>,
-                        (const void*)k_emf_ct<3, 1>, (const void*)k_emf_ct<3, 2>, (const void*)k_emf_ct<3, 3>};
-    for (const void* f : m) {
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EmfCtSmem));
-        if (e != cudaSuccess) return cuda_fail(c, e, "cudaFuncSetAttribute(EMF tile smem)");
     }
     return CUMC_OK;
 }
@@ -706,10 +700,8 @@ void run_stage(cumc_ctx* c, const Box& b, int stage, int part = 0) {
         return;
     }
     if (split && part == 2) {  // the rest: the x and y sweeps of the ghost planes 0 and nz+1 first
-        sweep<0>(c, b, pr, 0, 1);
-        sweep<0>(c, b, pr, b.nz + 1, 1);
-        sweep<1>(c, b, pr, 0, 1);
-        sweep<1>(c, b, pr, b.nz + 1, 1);
+        sweep<0>(c, b, pr, 0, 2, b.nz + 1);
+        sweep<1>(c, b, pr, 0, 2, b.nz + 1);
     } else {
         sweep<0>(c, b, pr);
         sweep<1>(c, b, pr);
@@ -763,6 +755,13 @@ void rk_step(cumc_ctx* c, const Box& b) {
     run_stage(c, b, 3);
 }
 
+// rk_step with the next step's dt formed at stage 3
+void rk_step_dt(cumc_ctx* c, const Box& b) {
+    c->fuse_dt = true;
+    rk_step(c, b);
+    c->fuse_dt = false;
+}
+
 // The step of cumc_rungekutta. Its launches are the same every call (dt and the
 // state stay in their places on the device), so from the second call on they
 // go as one graph: on small boxes the host's launches took longer than the
@@ -776,9 +775,7 @@ int rk_step_host(cumc_ctx* c) {
         cudaGraph_t g;
         const long long before = c->launches;
         CUMC_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        c->fuse_dt = true;
-        rk_step(c, c->box);
-        c->fuse_dt = false;
+        rk_step_dt(c, c->box);
         c->rk_launches = c->launches - before;
         c->launches = before;
         CUMC_CHECK(cudaStreamEndCapture(c->stream, &g));
@@ -790,9 +787,7 @@ int rk_step_host(cumc_ctx* c) {
         }
     }
     if (plain) {
-        c->fuse_dt = true;
-        rk_step(c, c->box);
-        c->fuse_dt = false;
+        rk_step_dt(c, c->box);
     } else {
         CUMC_CHECK(cudaGraphLaunch(c->rk_exec, c->stream));
         c->launches += c->rk_launches;
@@ -835,9 +830,7 @@ void loop_step(cumc_ctx* c, double t_end) {
     const Clock k = make_clock(c);
     launch(c, -1, 1, 1, k_step_begin, k, t_end);
     b.skip = k.done;
-    c->fuse_dt = true;
-    rk_step(c, b);
-    c->fuse_dt = false;
+    rk_step_dt(c, b);
     launch(c, -1, 1, 1, k_advance_time, k);
 }
 
@@ -1546,8 +1539,8 @@ int cumc_advance(cumc_ctx* c, int nsteps, double t_end, double* t_inout, int* st
             cudaGraph_t g;
             CUMC_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             const long long before = c->launches;
-            loop_step(c, t_end);
-            const long long per_step = c->launches - before;
+                loop_step(c, t_end);
+                const long long per_step = c->launches - before;
             c->launches = before;
             CUMC_CHECK(cudaStreamEndCapture(c->stream, &g));
             cudaError_t e = cudaGraphInstantiate(&c->graph_exec, g, 0);
@@ -1764,8 +1757,8 @@ void adj_sweeps(cumc_ctx* c, const Box& b, const Prim& pr, const AdjStage& st, c
         int nseg;
         const int seg = walk_segment_for<D>(b, WalkGeom<D>::ncols(b), c->sm_count, &nseg);
         const dim3 grid((unsigned)((WalkGeom<D>::ncols(b) + WK_THREADS - 1) / WK_THREADS), (unsigned)nseg);
-        launch_grid(c, -1, grid, WK_THREADS, walk_smem<double>(D), k_sweep_walk_sm<D, RECON, double, true>, b, c->tabs,
-                    pr, c->ggas, sl, seg, sr, 0, -1);
+        launch_grid(c, -1, grid, WK_THREADS, walk_smem<double>(D, RECON == 4), k_sweep_walk_sm<D, RECON, double, true>, b, c->tabs,
+                    pr, c->ggas, sl, seg, sr, 0, -1, 1);
     };
     // x: pass A per face, pass B one lane per cell and field
     launch(c, -1, xwarp_threads(b), 128, k_sweep_xwarp<RECON, double, true>, b, c->tabs, pr, c->ggas, sl, sr, 0, -1);
@@ -1783,8 +1776,7 @@ void adj_sweeps(cumc_ctx* c, const Box& b, const Prim& pr, const AdjStage& st, c
 
 // boundary^T: gather onto the sources, then clear the ghosts
 void adj_boundary(cumc_ctx* c, const Box& b, const BoundArgs& fw, const AdjPrim& lp, double* const* lbf) {
-    launch(c, -1, (long long)(b.nx + 1) * (b.ny + 1) * (b.nz + 1), 256, k_adj_boundary_gather, b, fw, lp, lbf[0],
-           lbf[1], lbf[2]);
+    launch(c, -1, face_set_cells(b), 256, k_adj_boundary_gather, b, fw, lp, lbf[0], lbf[1], lbf[2]);
     launch(c, -1, ghost_count(b), 256, k_adj_boundary_clear, b, fw, lp, lbf[0], lbf[1], lbf[2]);
 }
 

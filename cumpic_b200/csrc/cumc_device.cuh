@@ -143,6 +143,47 @@ __device__ __forceinline__ R tvd_slope(R vm, R vc, R vp, R cf, R cb) {
     return (R(0.5) * (copysign(R(1), dqf) + copysign(R(1), dqb))) * fmin(fabs(dqf), fabs(dqb));
 }
 
+// The reconstruction weights of one cell and its upper face, read (and, in the
+// mixed form, rounded to FP32) once for the seven fields: the sweeps store
+// between fields, so the compiler would read them again for each.
+template <int RECON, typename R>
+struct CellWeights {  // PPM: slope weights of cell c, interface weights of the face c | c+1
+    R s0, s1, a0, a1, a2, a3;
+    __device__ __forceinline__ CellWeights(const AxisTabs& A, int cs, int cf)
+        : s0((R)A.s0[cs]), s1((R)A.s1[cs]), a0((R)A.a0[cf]), a1((R)A.a1[cf]), a2((R)A.a2[cf]), a3((R)A.a3[cf]) {}
+    __device__ __forceinline__ R slope(R vm, R vc, R vp) const { return ppm_slope(vm, vc, vp, s0, s1); }
+    __device__ __forceinline__ R face(R vc, R vp, R dmc, R dmp) const {
+        return ppm_face(vc, vp, dmc, dmp, a0, a1, a2, a3);
+    }
+};
+template <typename R>
+struct CellWeights<1, R> {  // TVD
+    R cf, cb;
+    __device__ __forceinline__ CellWeights(const AxisTabs& A, int c) : cf((R)A.tcf[c]), cb((R)A.tcb[c]) {}
+    __device__ __forceinline__ R slope(R vm, R vc, R vp) const { return tvd_slope(vm, vc, vp, cf, cb); }
+};
+// TVD in FP64: the quotients by cf and cb share their reciprocals over the
+// fields (cumc_round.cuh; the plain operators outside the range)
+template <>
+struct CellWeights<1, double> {
+    double cf, cb;
+    Recip rf, rb;
+    bool ok;
+    __device__ __forceinline__ CellWeights(const AxisTabs& A, int c) : cf(A.tcf[c]), cb(A.tcb[c]) {
+        ok = range_max(cf, range_max(cb, 0u)) < RANGE_SPAN;
+        rf = recip_of(cf);
+        rb = recip_of(cb);
+    }
+    __device__ __forceinline__ double slope(double vm, double vc, double vp) const {
+        const double nf = 2.0 * (vp - vc), nb = 2.0 * (vc - vm);
+        if (!ok || tiny_min(nf, tiny_min(nb, ~0u)) < TINY) return tvd_slope(vm, vc, vp, cf, cb);
+        const double dqf = quot_signed(nf, cf, rf), dqb = quot_signed(nb, cb, rb);
+        // (sign(dqf) + sign(dqb))/2 min(|dqf|, |dqb|), a zero positive where the signs differ
+        const bool same = (__double2hiint(dqf) >= 0) == (__double2hiint(dqb) >= 0);
+        return same ? copysign(min_mag(fabs(dqf), fabs(dqb)), dqf) : 0.0;
+    }
+};
+
 // ---------------------------------------------------------------------------
 // HLL Riemann solver at one face (solver/rsolver.f90:43-130)
 // ---------------------------------------------------------------------------
@@ -165,6 +206,17 @@ __device__ __forceinline__ R signalspeed(R cs, R bn, R bt1, R bt2, R rho) {
 // the IEEE operations
 __device__ __forceinline__ double recip_r(double x) { return recip_near(x, recip_seed(x)); }
 __device__ __forceinline__ float recip_r(float x) { return 1.0f / x; }
+// FP32 with (ROUNDED) and without the branch-free forms: the same values where
+// hll_flux7_mixed's range test holds
+template <bool ROUNDED>
+__device__ __forceinline__ float recip_q(float x) { return ROUNDED ? recip_f(x) : 1.0f / x; }
+template <bool ROUNDED>
+__device__ __forceinline__ float root_q(float x) { return ROUNDED ? root_f(x) : sqrtf(x); }
+template <bool ROUNDED>
+__device__ __forceinline__ float root_max0_q(float x) {
+    if (!ROUNDED) return sqrtf(fmaxf(x, 0.0f));
+    return x > 0.0f ? root_f(x) : 0.0f;
+}
 __device__ __forceinline__ double sqrt_r(double x) { return root_pos(x); }
 __device__ __forceinline__ float sqrt_r(float x) { return sqrtf(x); }
 __device__ __forceinline__ double sqrt_max0(double x) { return root_pos(x); }
@@ -542,21 +594,42 @@ __device__ __forceinline__ SideScalars side_scalars64(const float (&w)[8], float
     return {rho * (e + 0.5 * vsq) + 0.5 * bsq, 0.5 * bsq, (bx * vx + by * vy) + bz * vz};
 }
 
-template <int DIR>
-__device__ __forceinline__ void hll_flux7_mixed(const float (&wl)[8], const float (&wr)[8], float ggas,
-                                                float (&out)[7]) {
+// signalspeed_recip in FP32 with the roots' form chosen
+template <bool ROUNDED>
+__device__ __forceinline__ float signalspeed_q(float cs, float bn, float bt1, float bt2, float irho) {
+    const float a2 = cs * cs;
+    const float a4 = a2 * a2;
+    const float b2n = (bn * bn) * irho;
+    const float b2t1 = (bt1 * bt1) * irho;
+    const float b2t2 = (bt2 * bt2) * irho;
+    const float b2 = (b2n + b2t1) + b2t2;
+    const float b4 = b2 * b2;
+    return root_q<ROUNDED>(
+        0.5f * ((a2 + b2) + root_max0_q<ROUNDED>(((a4 + b4) + (2.0f * b2) * a2) - (4.0f * a2) * b2n)));
+}
+
+// ROUNDED: the five FP32 reciprocals and eight roots without their range
+// branches; false (nothing computed) where a density leaves [2^-60, 2^60) or
+// gamma p/rho leaves [2^-38, 2^45)
+template <int DIR, bool ROUNDED>
+__device__ __forceinline__ bool hll_flux7_mixed_form(const float (&wl)[8], const float (&wr)[8], float ggas,
+                                                     float (&out)[7]) {
     constexpr int ivn = IVX + DIR;
     constexpr int ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
     constexpr int HYDRO = 5;  // components 0..4 in FP64
-    const float irL = 1.0f / wl[IRHO], irR = 1.0f / wr[IRHO];
+    const float irL = recip_q<ROUNDED>(wl[IRHO]), irR = recip_q<ROUNDED>(wr[IRHO]);
     float sL, sR;
     {
-        const float csL = sqrtf((ggas * wl[ITAU]) * irL);
-        const float csR = sqrtf((ggas * wr[ITAU]) * irR);
-        const float cfsL = signalspeed_recip<float>(csL, wl[ibn], wl[ibt1], wl[ibt2], irL);
-        const float cfsR = signalspeed_recip<float>(csR, wr[ibn], wr[ibt1], wr[ibt2], irR);
-        const float sqL = sqrtf(wl[IRHO]), sqR = sqrtf(wr[IRHO]);
-        const float isq = 1.0f / (sqL + sqR);
+        const float xL = (ggas * wl[ITAU]) * irL, xR = (ggas * wr[ITAU]) * irR;
+        if (ROUNDED && (range_max_f<-60>(wl[IRHO], range_max_f<-60>(wr[IRHO], 0u)) >= 120u << 23 ||
+                        range_max_f<-38>(xL, range_max_f<-38>(xR, 0u)) >= 83u << 23))
+            return false;
+        const float csL = root_q<ROUNDED>(xL);
+        const float csR = root_q<ROUNDED>(xR);
+        const float cfsL = signalspeed_q<ROUNDED>(csL, wl[ibn], wl[ibt1], wl[ibt2], irL);
+        const float cfsR = signalspeed_q<ROUNDED>(csR, wr[ibn], wr[ibt1], wr[ibt2], irR);
+        const float sqL = root_q<ROUNDED>(wl[IRHO]), sqR = root_q<ROUNDED>(wr[IRHO]);
+        const float isq = recip_q<ROUNDED>(sqL + sqR);
         const float ubar = (sqL * wl[ivn] + sqR * wr[ivn]) * isq;
         const float cbar = (sqL * cfsL + sqR * cfsR) * isq;
         sL = fminf(wl[ivn] - cfsL, ubar - cbar);
@@ -577,7 +650,9 @@ __device__ __forceinline__ void hll_flux7_mixed(const float (&wl)[8], const floa
         for (int q = 0; q < 7; ++q)
             out[q] = q < HYDRO ? (float)side_f<double>(L, comp[q], aL.E, aL.hb2, aL.vdotb) : L.f(comp[q]);
     } else if (sR >= 0.0f) {
-        const float idsf = 1.0f / (sR - sL), lrf = sL * sR;
+        // sR - sL > 0 is at least a sound speed, 2^-19
+        const float ds = sR - sL, lrf = sL * sR;
+        const float idsf = ROUNDED && ds < 0x1p100f ? recip_q<ROUNDED>(ds) : 1.0f / ds;
         const double cl = sL, cr = sR, ids = rcp_newton(cr - cl, idsf), lr = cl * cr;
 #pragma unroll
         for (int q = 0; q < 7; ++q) {
@@ -596,7 +671,35 @@ __device__ __forceinline__ void hll_flux7_mixed(const float (&wl)[8], const floa
         for (int q = 0; q < 7; ++q)
             out[q] = q < HYDRO ? (float)side_f<double>(Rs, comp[q], aR.E, aR.hb2, aR.vdotb) : Rs.f(comp[q]);
     }
+    return true;
 }
+
+// the plain form out of line
+template <int DIR>
+__device__ __noinline__ void hll_flux7_mixed_plain(const float* w, float ggas, float* out) {
+    float wl[8], wr[8], fx[7];
+    for (int q = 0; q < 8; ++q) {
+        wl[q] = w[q];
+        wr[q] = w[8 + q];
+    }
+    hll_flux7_mixed_form<DIR, false>(wl, wr, ggas, fx);
+    for (int q = 0; q < 7; ++q) out[q] = fx[q];
+}
+template <int DIR>
+__device__ __forceinline__ void hll_flux7_mixed(const float (&wl)[8], const float (&wr)[8], float ggas,
+                                                float (&out)[7]) {
+    if (hll_flux7_mixed_form<DIR, true>(wl, wr, ggas, out)) return;
+    float w[16], f[7];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        w[q] = wl[q];
+        w[8 + q] = wr[q];
+    }
+    hll_flux7_mixed_plain<DIR>(w, ggas, f);
+#pragma unroll
+    for (int q = 0; q < 7; ++q) out[q] = f[q];
+}
+
 
 // the sweeps' HLL solve: hll_flux7 in FP64 (RECIP: the CUMC_FP64_FAST form).
 // For the mixed form's float states, RECIP selects the all-FP32 reciprocal

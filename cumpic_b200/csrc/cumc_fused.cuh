@@ -311,12 +311,13 @@ __global__ void __launch_bounds__(WK_THREADS) k_walk_acc(Box b, Tabs T, Prim pr,
     for (int f = f0; f < f1; ++f) {
         double wl[8], wr[8];
         const double bn = bnp[f * s];
+        const auto cw = walk_weights<RECON, double>(A, f);
 #pragma unroll
         for (int v = 0; v < WK_FIELDS; ++v) {
             const double x = nxt[v];
             double d1 = at(3, v), Vf = at(4, v);
             double vm1, vp1;
-            walk_step<RECON>(A, f, RECON == 4 ? 0.0 : at(r0, v), at(r1, v), at(r2, v), x, d1, Vf, vm1, vp1);
+            walk_step<RECON>(cw, RECON == 4 ? 0.0 : at(r0, v), at(r1, v), at(r2, v), x, d1, Vf, vm1, vp1);
             wl[slot[v]] = at(5, v);  // vp_out of cell f
             wr[slot[v]] = vm1;       // vm_out of cell f+1
             at(5, v) = vp1;

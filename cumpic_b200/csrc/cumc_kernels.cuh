@@ -49,11 +49,11 @@ __global__ void __launch_bounds__(128) k_sweep(Box b, Tabs T, PrimT<R> pr, R gga
     const int n1 = (DIR == 1 ? b.ny : b.ny + 1) + 1;
     const int n2 = (DIR == 2 ? b.nz : b.nz + 1) + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total || (b.skip && *b.skip)) return;
     const int j = (int)(t % n0);
     const int k = (int)((t / n0) % n1);
-    const int l = (int)(t / ((long long)n0 * n1));
+    const int l = (int)(t / n0 / n1);
     const int base = b.idx(j, k, l);
     const int s = DIR == 0 ? 1 : DIR == 1 ? b.SX : b.SX * b.SY;
     const int c = DIR == 0 ? j : DIR == 1 ? k : l;  // face between cell c and c+1
@@ -130,11 +130,11 @@ __global__ void __launch_bounds__(256) k_emf(Box b, PrimT<R> pr, FaceFluxT<R> fx
                                              EdgeET<R> out) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total || (b.skip && *b.skip)) return;
     const int j = (int)(t % n0);
     const int k = (int)((t / n0) % n1);
-    const int l = (int)(t / ((long long)n0 * n1));
+    const int l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     const int sj = 1, sk = b.SX, sl = b.SX * b.SY;
     // x-faces carry (by, bz) fluxes, y-faces (bx, bz), z-faces (bx, by)
@@ -324,11 +324,11 @@ __device__ __forceinline__ double rk_point(double u0, double uc, double dt, doub
 __device__ __forceinline__ bool box1_index(const Box& b, int& j, int& k, int& l, int& i) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total || (b.skip && *b.skip)) return false;
     j = (int)(t % n0);
     k = (int)((t / n0) % n1);
-    l = (int)(t / ((long long)n0 * n1));
+    l = (int)(t / n0 / n1);
     i = b.idx(j, k, l);
     return true;
 }
@@ -660,13 +660,15 @@ __global__ void __launch_bounds__(256, CUMC_COMB_MINB) k_combine_utop2(Box b, Ta
                                                                         UtopArgs o) {
     if (b.skip && *b.skip) return;
     const int np = (b.nx + 2) >> 1, n1 = b.ny + 1, n2 = b.nz + 1;
+    // (64-bit index: with 32-bit divisions this kernel, which waits on DRAM,
+    // measured 2-5 % slower)
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = t < (long long)np * n1 * n2;
     const bool fuse_dt = STAGE == 3 && o.dtmin;
     if (!live && !fuse_dt) return;
     double dt_cell = 1.0e10;
     if (live) {
-        const int j = (int)(t % np) * 2, k = (int)((t / np) % n1), l = (int)(t / ((long long)np * n1));
+        const int j = (int)(t % np) * 2, k = (int)((t / np) % n1), l = (int)(t / np / n1);
         const int i = b.idx(j, k, l);
         const int sk = b.SX, sl = b.SX * b.SY;
         const bool two = j + 1 <= b.nx;
@@ -821,19 +823,22 @@ using BoundArgs = BoundArgsT<double>;
 
 template <int MODEL, typename R>
 __global__ void __launch_bounds__(256) k_boundary(Box b, BoundArgsT<R> a) {
-    const long long zsl = 6LL * b.SX * b.SY, ysl = 6LL * b.SX * b.nz, xsl = 6LL * b.ny * b.nz;
+    // 32-bit index arithmetic: a box has fewer than 2^31 cells (cumc_init), and
+    // 64-bit divisions cost more than the copies
+    const unsigned zp = (unsigned)b.SX * b.SY, yp = (unsigned)b.SX * b.nz;
+    const unsigned zsl = 6u * zp, ysl = 6u * yp, xsl = 6u * b.ny * b.nz;
     if (b.skip && *b.skip) return;
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     int j, k, l;
     if (t < zsl) {
-        const int s = (int)(t / ((long long)b.SX * b.SY));
-        const int r = (int)(t % ((long long)b.SX * b.SY));
+        const int s = (int)(t / zp);
+        const int r = (int)(t % zp);
         l = s < 3 ? s - 2 : b.nz + s - 2;
         k = r / b.SX - 2;
         j = r % b.SX - 2;
     } else if ((t -= zsl) < ysl) {
-        const int s = (int)(t / ((long long)b.SX * b.nz));
-        const int r = (int)(t % ((long long)b.SX * b.nz));
+        const int s = (int)(t / yp);
+        const int r = (int)(t % yp);
         k = s < 3 ? s - 2 : b.ny + s - 2;
         l = r / b.SX + 1;
         j = r % b.SX - 2;
@@ -841,7 +846,7 @@ __global__ void __launch_bounds__(256) k_boundary(Box b, BoundArgsT<R> a) {
         // the six x ghosts of a row on six consecutive threads, so that a warp
         // reads and writes a few row segments instead of 32 rows
         const int s = (int)(t % 6);
-        const long long r = t / 6;
+        const unsigned r = t / 6;
         j = s < 3 ? s - 2 : b.nx + s - 2;
         l = (int)(r / b.ny) + 1;
         k = (int)(r % b.ny) + 1;
@@ -936,12 +941,12 @@ __global__ void __launch_bounds__(256) k_finddt(Box b, Tabs T, PrimT<R> pr, doub
                                                 unsigned long long* dtmin) {
     if (b.skip && *b.skip) return;
     const long long total = (long long)b.nx * b.ny * b.nz;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     double dt_out = 1.0e10;
     if (t < total) {
         const int j = (int)(t % b.nx) + 1;
         const int k = (int)((t / b.nx) % b.ny) + 1;
-        const int l = (int)(t / ((long long)b.nx * b.ny)) + 1;
+        const int l = (int)(t / b.nx / b.ny) + 1;
         const int i = b.idx(j, k, l);
         dt_out = cell_dt<COORD>(T, j, k, l, pr.w[0][i], (double)pr.w[4][i], pr.w[1][i], pr.w[2][i], pr.w[3][i],
                                 pr.bc[0][i], pr.bc[1][i], pr.bc[2][i], ggas, cfl);
@@ -1010,12 +1015,12 @@ template <int COORD>
 __global__ void __launch_bounds__(256) k_divb(Box b, Tabs T, const double* bx, const double* by, const double* bz,
                                               double* part) {
     const long long total = (long long)b.nx * b.ny * b.nz;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     double smax = -1.0e300, amax = 0.0, fmaxv = 0.0;
     if (t < total) {
         const int j = (int)(t % b.nx) + 1;
         const int k = (int)((t / b.nx) % b.ny) + 1;
-        const int l = (int)(t / ((long long)b.nx * b.ny)) + 1;
+        const int l = (int)(t / b.nx / b.ny) + 1;
         const int i = b.idx(j, k, l);
         const double dxl = T.ax[0].d[j], dyl = T.ax[1].d[k], dzl = T.ax[2].d[l];
         double axp, axm, ayp, aym, azp, azm;

@@ -167,11 +167,11 @@ __global__ void __launch_bounds__(256, CUMC_MXC_MINB) k_combine_mx(Box b, Tabs T
                                                     FaceFluxT<float> fz, CombineMx a) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total || (b.skip && *b.skip)) return;
     const int j = (int)(t % n0);
     const int k = (int)((t / n0) % n1);
-    const int l = (int)(t / ((long long)n0 * n1));
+    const int l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     const int sj = 1, sk = b.SX, sl = b.SX * b.SY;
     float L[8];
@@ -353,11 +353,11 @@ struct UtopMx {
 // then stays to the block's min reduction.
 // one cell (flat index t on (0:n)^3); returns its CFL dt when fuse_dt, else 1e10
 template <int COORD, int MODEL, bool FINAL>
-__device__ __forceinline__ double utop_mx_cell(const Box& b, const Tabs& T, const UtopMx& a, long long t, bool fuse_dt) {
+__device__ __forceinline__ double utop_mx_cell(const Box& b, const Tabs& T, const UtopMx& a, unsigned t, bool fuse_dt) {
     const int n0 = b.nx + 1, n1 = b.ny + 1;
     const int j = (int)(t % n0);
     const int k = (int)((t / n0) % n1);
-    const int l = (int)(t / ((long long)n0 * n1));
+    const int l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     const bool interior = j >= 1 && k >= 1 && l >= 1;
     auto U = [&](int q, int at) -> double {
@@ -433,7 +433,7 @@ __device__ __forceinline__ double utop_mx_cell(const Box& b, const Tabs& T, cons
 template <int COORD, int MODEL, bool FINAL>
 __global__ void __launch_bounds__(256, CUMC_MXU_MINB) k_utop_mx(Box b, Tabs T, UtopMx a) {
     const long long total = (long long)(b.nx + 1) * (b.ny + 1) * (b.nz + 1);
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (b.skip && *b.skip) return;  // the same for every thread
     const bool fuse_dt = FINAL && a.dtmin;
     if (t >= total && !fuse_dt) return;
@@ -457,6 +457,8 @@ __global__ void __launch_bounds__(256, CUMC_CUMX_MINB) k_combine_utop_mx(Box b, 
     constexpr bool FINAL = STAGE == 3;
     const int n0 = b.nx + 1, n1 = b.ny + 1;
     const long long total = (long long)n0 * n1 * (b.nz + 1);
+    // (64-bit index: with 32-bit divisions this kernel, which waits on DRAM,
+    // measured 2-5 % slower)
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (b.skip && *b.skip) return;
     const bool fuse_dt = FINAL && a.dtmin;
@@ -465,7 +467,7 @@ __global__ void __launch_bounds__(256, CUMC_CUMX_MINB) k_combine_utop_mx(Box b, 
     if (t < total) {
         const int j = (int)(t % n0);
         const int k = (int)((t / n0) % n1);
-        const int l = (int)(t / ((long long)n0 * n1));
+        const int l = (int)(t / n0 / n1);
         const int i = b.idx(j, k, l);
         const bool interior = j >= 1 && k >= 1 && l >= 1;
         float L[5];
@@ -580,11 +582,11 @@ __global__ void __launch_bounds__(256) k_initial_mx(Box b, UtopMx a, const doubl
                                                     const double* __restrict__ eps) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
     const int j = (int)(t % n0);
     const int k = (int)((t / n0) % n1);
-    const int l = (int)(t / ((long long)n0 * n1));
+    const int l = (int)(t / n0 / n1);
     const int i = b.idx(j, k, l);
     const bool interior = j >= 1 && k >= 1 && l >= 1;
     const int off[3] = {1, b.SX, b.SX * b.SY};
@@ -667,14 +669,14 @@ void sweep_mx(const Launcher& L, const Box& b, const Tabs& T, const PrimT<float>
         int nseg;
         const int seg = walk_segment_for<D>(b, WalkGeom<D>::ncols(b), sm_count, &nseg);
         const dim3 grid((unsigned)((WalkGeom<D>::ncols(b) + WK_THREADS - 1) / WK_THREADS), (unsigned)nseg);
-        const size_t sm = walk_smem<float>(D);
+        const size_t sm = walk_smem<float>(D, ppm);
         if (fp32)
             run(L, DIR, grid, WK_THREADS, sm,
                 ppm ? k_sweep_walk_sm<D, 4, float, false, true> : k_sweep_walk_sm<D, 1, float, false, true>, b, T, pr,
-                ggas, out, seg, out, 0, -1);
+                ggas, out, seg, out, 0, -1, 1);
         else
             run(L, DIR, grid, WK_THREADS, sm, ppm ? k_sweep_walk_sm<D, 4, float> : k_sweep_walk_sm<D, 1, float>, b, T,
-                pr, ggas, out, seg, out, 0, -1);
+                pr, ggas, out, seg, out, 0, -1, 1);
         return;
     }
     // x: one lane per cell

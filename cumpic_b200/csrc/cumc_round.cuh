@@ -149,6 +149,26 @@ __device__ __forceinline__ void quot_group(const double (&a)[N], double b, doubl
         for (int n = 0; n < N; ++n) q[n] = plain_quot(a[n], b);
     }
 }
+
+// FP32 reciprocal and root, rounded to nearest (the results of 1.0f/x and
+// sqrtf, checked over every significand by the tests): one Newton step from
+// the hardware's approximation and the remainder correction. x in 2^+-100.
+__device__ __forceinline__ float recip_f(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+}
+__device__ __forceinline__ float root_f(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float g = x * y;
+    return __fmaf_rn(__fmaf_rn(-g, g, x), 0.5f * y, g);
+}
+// max(bits - bits of 2^LO), as range_max: below `span << 23` for x in [2^LO, 2^(LO + span))
+template <int LO>
+__device__ __forceinline__ unsigned range_max_f(float x, unsigned m) {
+    return __viaddmax_u32(__float_as_uint(x), 0u - ((unsigned)(127 + LO) << 23), m);
+}
 #endif
 
 }  // namespace cumc

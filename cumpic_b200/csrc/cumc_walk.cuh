@@ -63,7 +63,10 @@ struct WalkGeom {
 // 8 while the grid gave fewer than 32 warps a SM: 64^3 0.036 -> 0.029 ms a
 // walk, the 90x26x75 torus 0.029 -> 0.023, a 512x4x4 tube 0.021 -> 0.013; 256^3
 // unchanged (0.90).
-constexpr int WK_RESIDENT = 10;
+#ifndef CUMC_WALK_RES
+#define CUMC_WALK_RES 10
+#endif
+constexpr int WK_RESIDENT = CUMC_WALK_RES;
 template <int DIR>
 inline int walk_segment_for(const Box& b, long long ncols, int sm_count, int* nseg) {
     const int faces = WalkGeom<DIR>::nd(b) + 1;
@@ -95,7 +98,8 @@ __device__ __forceinline__ int walk_base(const Box& b, long long col) {
 // column set-up shared by both window forms. Every thread of a block stays
 // to the end (the x sweep synchronises the block); threads past the last
 // column walk a copy of it and store nothing. The columns are those whose
-// slow transverse index lies in c_lo .. c_lo + c_cnt - 1 (c_cnt < 0: all).
+// slow transverse index is c_lo, c_lo + c_step, .. (c_cnt of them; c_cnt < 0:
+// all).
 template <int DIR, typename R>
 struct WalkCol {
     int base, s, f0, f1, nd;
@@ -103,7 +107,7 @@ struct WalkCol {
     const R* src[WK_FIELDS];
     int slot[WK_FIELDS];
     const R* bn;
-    __device__ bool init(const Box& b, const PrimT<R>& pr, int seg, int c_lo = 0, int c_cnt = -1) {
+    __device__ bool init(const Box& b, const PrimT<R>& pr, int seg, int c_lo = 0, int c_cnt = -1, int c_step = 1) {
         using G = WalkGeom<DIR>;
         if (b.skip && *b.skip) return false;
         if (c_cnt < 0) c_cnt = G::wc(b);
@@ -115,8 +119,8 @@ struct WalkCol {
         if (f0 > nd) return false;
         f1 = min(f0 + seg, nd + 1);
         s = G::stride(b);
-        const long long cc = min(col, ncols - 1);
-        base = G::idx(b, (int)(cc % G::wa(b)), c_lo + (int)(cc / G::wa(b)), 0);
+        const unsigned cc = (unsigned)min(col, ncols - 1);  // fewer columns than cells: 32-bit division
+        base = G::idx(b, (int)(cc % G::wa(b)), c_lo + c_step * (int)(cc / G::wa(b)), 0);
         // tangential cell fields: (by, bz) for x, (bx, bz) for y, (bx, by) for z
         constexpr int ta = DIR == 0 ? 1 : 0;
         constexpr int tb = DIR == 2 ? 1 : 2;
@@ -223,20 +227,28 @@ __device__ __forceinline__ void walk_prologue(const AxisTabs& A, int f0, R x0, R
     }
 }
 
+// the weights of the step at face f: PPM forms the slope of cell f+2 and the
+// interface value between f+1 and f+2, TVD the slope of cell f+1
+template <int RECON, typename R>
+__device__ __forceinline__ CellWeights<RECON, R> walk_weights(const AxisTabs& A, int f) {
+    if constexpr (RECON == 4) return CellWeights<RECON, R>(A, f + 2, f + 1);
+    else return CellWeights<RECON, R>(A, f + 1);
+}
+
 // one window step for one field at face f: from v(f) (TVD), v(f+1), v(f+2),
 // the new cell x = v(f+3), the carried slope d1 and interface Vf, returns
 // vm_out(f+1), vp_out(f+1) and updates d1, Vf
 template <int RECON, typename R>
-__device__ __forceinline__ void walk_step(const AxisTabs& A, int f, R v0, R v1, R v2, R x, R& d1, R& Vf, R& vm1,
+__device__ __forceinline__ void walk_step(const CellWeights<RECON, R>& W, R v0, R v1, R v2, R x, R& d1, R& Vf, R& vm1,
                                           R& vp1) {
-    if (RECON == 4) {
-        const R d2 = ppm_slope(v1, v2, x, (R)A.s0[f + 2], (R)A.s1[f + 2]);
-        const R Vn = ppm_face(v1, v2, d1, d2, (R)A.a0[f + 1], (R)A.a1[f + 1], (R)A.a2[f + 1], (R)A.a3[f + 1]);
+    if constexpr (RECON == 4) {
+        const R d2 = W.slope(v1, v2, x);
+        const R Vn = W.face(v1, v2, d1, d2);
         ppm_fix(v1, Vf, Vn, vm1, vp1);
         d1 = d2;
         Vf = Vn;
     } else {
-        const R sl = tvd_slope(v0, v1, v2, (R)A.tcf[f + 1], (R)A.tcb[f + 1]);
+        const R sl = W.slope(v0, v1, v2);
         vm1 = v1 - R(0.5) * sl;
         vp1 = v1 + R(0.5) * sl;
     }
@@ -307,11 +319,12 @@ __global__ void __launch_bounds__(WK_THREADS, 5) k_sweep_walk(Box b, Tabs T, Pri
         const int j = (f - f0) & (XS_CELLS - 1);
         if (DIR == 0 && j == 0) walk_chunk(C, f, X, out);
         const R bn = DIR == 0 ? X.get(WK_FIELDS, j) : C.bn[f * s];
+        const auto W = walk_weights<RECON, R>(A, f);
 #pragma unroll
         for (int v = 0; v < WK_FIELDS; ++v) {
             const R x = nxt[v];
             R vm1, vp1;
-            walk_step<RECON>(A, f, v0[v], v1[v], v2[v], x, d1[v], Vf[v], vm1, vp1);
+            walk_step<RECON>(W, v0[v], v1[v], v2[v], x, d1[v], Vf[v], vm1, vp1);
             wl[C.slot[v]] = vpf[v];  // vp_out of cell f
             wr[C.slot[v]] = vm1;     // vm_out of cell f+1
             vpf[v] = vp1;
@@ -329,36 +342,44 @@ __global__ void __launch_bounds__(WK_THREADS, 5) k_sweep_walk(Box b, Tabs T, Pri
     if (DIR == 0) walk_last(C, X, out);
 }
 
-// shared-memory window: slots 0..2 are a ring of cell values (v(c) in slot
-// c mod 3), 3 the carried slope, 4 the carried interface value, 5 vp_out(f)
-constexpr int WK_SLOTS = 6;
+// shared-memory window. PPM steps from v(f+1), v(f+2), the carried slope and
+// interface value: a ring of two cell values and three slots; TVD from v(f),
+// v(f+1), v(f+2): a ring of three and one slot. The last slot is vp_out(f).
+template <int RECON>
+struct WalkSlots {
+    static constexpr int RING = RECON == 4 ? 2 : 3, D1 = RING, VF = RING + 1, VP = RECON == 4 ? RING + 2 : RING,
+                         COUNT = VP + 1;
+};
 template <typename R>
-constexpr size_t walk_smem(int dir) {
-    return (size_t)WK_SLOTS * WK_FIELDS * WK_THREADS * sizeof(R) + (dir == 0 ? xstage_smem<R>() : 0);
+inline size_t walk_smem(int dir, bool ppm) {
+    return (size_t)(ppm ? WalkSlots<4>::COUNT : WalkSlots<1>::COUNT) * WK_FIELDS * WK_THREADS * sizeof(R) +
+           (dir == 0 ? xstage_smem<R>() : 0);
 }
+constexpr int WK_SLOTS = 6;  // slots of the fused walkers (cumc_fused.cuh): a ring of three, slope, interface, vp_out
 
 // STATES (y and z only): instead of solving HLL, store each face's
 // reconstructed states, left in out and right in out_r (field order of the
 // sweep, at the face's left cell), for the adjoint's HLL transpose.
-// c_lo, c_cnt: the columns walked (WalkCol; c_cnt < 0 for all)
+// c_lo, c_cnt, c_step: the columns walked (WalkCol; c_cnt < 0 for all)
 // RECIP: the HLL solve's quotients as products with reciprocals (hll_flux7)
 template <int DIR, int RECON, typename R, bool STATES = false, bool RECIP = false>
 __global__ void __launch_bounds__(WK_THREADS, CUMC_WALK_MINB) k_sweep_walk_sm(Box b, Tabs T, PrimT<R> pr, R ggas, FaceFluxT<R> out,
-                                                             int seg, FaceFluxT<R> out_r, int c_lo, int c_cnt) {
+                                                             int seg, FaceFluxT<R> out_r, int c_lo, int c_cnt, int c_step) {
     static_assert(!STATES || DIR != 0, "face states along y and z");
     extern __shared__ __align__(16) unsigned char wk_raw[];
     R* const sm = reinterpret_cast<R*>(wk_raw) + threadIdx.x;
     auto at = [&](int slot, int v) -> R& { return sm[(slot * WK_FIELDS + v) * WK_THREADS]; };
     WalkCol<DIR, R> C;
-    if (!C.init(b, pr, seg, c_lo, c_cnt)) return;
+    if (!C.init(b, pr, seg, c_lo, c_cnt, c_step)) return;
     const AxisTabs A = T.ax[DIR];
     const int s = C.s, f0 = C.f0;
     XStage<R> X;
-    if (DIR == 0) X.init(b, pr, reinterpret_cast<R*>(wk_raw) + WK_SLOTS * WK_FIELDS * WK_THREADS);
+    using W = WalkSlots<RECON>;
+    if (DIR == 0) X.init(b, pr, reinterpret_cast<R*>(wk_raw) + W::COUNT * WK_FIELDS * WK_THREADS);
 
     R nxt[WK_FIELDS];
-    // ring positions of v(f), v(f+1), v(f+2) for f = f0
-    int r0 = f0 % 3, r1 = (f0 + 1) % 3, r2 = (f0 + 2) % 3;
+    // ring positions of v(f), v(f+1), v(f+2) for f = f0 (a ring of two has no v(f))
+    int r0 = f0 % W::RING, r1 = (f0 + 1) % W::RING, r2 = (f0 + 2) % W::RING;
 #pragma unroll
     for (int v = 0; v < WK_FIELDS; ++v) {
         const R* q = C.src[v];
@@ -366,12 +387,14 @@ __global__ void __launch_bounds__(WK_THREADS, CUMC_WALK_MINB) k_sweep_walk_sm(Bo
                 x4 = q[(f0 + 2) * s];
         R vpf, d1, Vf;
         walk_prologue<RECON>(A, f0, x0, x1, x2, x3, x4, vpf, d1, Vf);
-        at(r0, v) = x2;
+        if (RECON != 4) at(r0, v) = x2;
         at(r1, v) = x3;
         at(r2, v) = x4;
-        at(3, v) = d1;
-        at(4, v) = Vf;
-        at(5, v) = vpf;
+        if (RECON == 4) {
+            at(W::D1, v) = d1;
+            at(W::VF, v) = Vf;
+        }
+        at(W::VP, v) = vpf;
         nxt[v] = q[(f0 + 3) * s];
     }
 
@@ -380,25 +403,32 @@ __global__ void __launch_bounds__(WK_THREADS, CUMC_WALK_MINB) k_sweep_walk_sm(Bo
         const int j = (f - f0) & (XS_CELLS - 1);
         if (DIR == 0 && j == 0) walk_chunk(C, f, X, out);
         const R bn = DIR == 0 ? X.get(WK_FIELDS, j) : C.bn[f * s];
+        const auto cw = walk_weights<RECON, R>(A, f);
 #pragma unroll
         for (int v = 0; v < WK_FIELDS; ++v) {
             const R x = nxt[v];
-            R d1 = at(3, v), Vf = at(4, v);
+            R d1 = RECON == 4 ? at(W::D1, v) : R(0), Vf = RECON == 4 ? at(W::VF, v) : R(0);
             R vm1, vp1;
-            walk_step<RECON>(A, f, RECON == 4 ? R(0) : at(r0, v), at(r1, v), at(r2, v), x, d1, Vf, vm1, vp1);
-            wl[C.slot[v]] = at(5, v);  // vp_out of cell f
-            wr[C.slot[v]] = vm1;       // vm_out of cell f+1
-            at(5, v) = vp1;
+            walk_step<RECON>(cw, RECON == 4 ? R(0) : at(r0, v), at(r1, v), at(r2, v), x, d1, Vf, vm1, vp1);
+            wl[C.slot[v]] = at(W::VP, v);  // vp_out of cell f
+            wr[C.slot[v]] = vm1;           // vm_out of cell f+1
+            at(W::VP, v) = vp1;
             if (RECON == 4) {
-                at(3, v) = d1;
-                at(4, v) = Vf;
+                at(W::D1, v) = d1;
+                at(W::VF, v) = Vf;
             }
-            at(r0, v) = x;  // v(f+3) replaces v(f)
+            at(RECON == 4 ? r1 : r0, v) = x;  // v(f+3) takes the place of the oldest value
         }
-        const int r = r0;
-        r0 = r1;
-        r1 = r2;
-        r2 = r;
+        if (RECON == 4) {
+            const int r = r1;
+            r1 = r2;
+            r2 = r;
+        } else {
+            const int r = r0;
+            r0 = r1;
+            r1 = r2;
+            r2 = r;
+        }
         if (f + 1 < C.f1) {
 #pragma unroll
             for (int v = 0; v < WK_FIELDS; ++v) nxt[v] = DIR == 0 ? X.get(v, j) : C.src[v][(f + 4) * s];
@@ -446,13 +476,13 @@ __global__ void __launch_bounds__(128, CUMC_XWARP_MINB) k_sweep_xwarp(Box b, Tab
                                                         FaceFluxT<R> out_r, int l_lo, int l_cnt) {
     constexpr unsigned FULL = 0xffffffffu;
     const int nw = (b.nx + 1 + XW_FACES - 1) / XW_FACES;  // warps per row
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const unsigned warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (l_cnt < 0) l_cnt = b.nz + 2;
     const long long rows = (long long)(b.ny + 2) * l_cnt;
     if (warp >= rows * nw || (b.skip && *b.skip)) return;  // uniform over the warp
     const int w = (int)(warp % nw);
-    const long long row = warp / nw;
+    const unsigned row = warp / nw;
     const int k = (int)(row % (b.ny + 2)), l = l_lo + (int)(row / (b.ny + 2));
     const int c = w * XW_FACES - 2 + lane;  // this lane's cell; its face is c | c+1
     const bool inb = c >= -2 && c <= b.nx + 3;
@@ -544,39 +574,45 @@ __device__ __forceinline__ void st_pair(R* p, int i, R a, R b, bool oka, bool ok
     }
 }
 
+// cell c's weights; TVD slopes count on 0..n+1 only, and beyond it the weights
+// of the nearest such cell keep them on the rounded path
+template <int RECON, typename R>
+__device__ __forceinline__ CellWeights<RECON, R> xpair_weights(const AxisTabs& A, int c, int n) {
+    if constexpr (RECON == 4) return CellWeights<RECON, R>(A, c, c);
+    else return CellWeights<RECON, R>(A, min(max(c, 0), n + 1));
+}
+
 template <int RECON, typename R, bool RECIP, bool VEC>
 __global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box b, Tabs T, PrimT<R> pr, R ggas,
-                                                                           FaceFluxT<R> out, int l_lo) {
+                                                                           FaceFluxT<R> out, int l_lo, int l_step) {
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ R sm[28][XP_THREADS];  // states of the pair's two faces: left 7, right 7 each
     const int cells = b.SX * (b.ny + 2);
     const int w = blockIdx.x * (XP_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31, tid = threadIdx.x;
     if (w * XP_FACES + 2 >= cells || (b.skip && *b.skip)) return;  // uniform over the warp
     const int m = w * XP_FACES + 2 * lane;  // position of the lane's first cell in the plane's line
-    const int g = b.idx(-2, 0, l_lo + (int)blockIdx.y) + m;
+    const int g = b.idx(-2, 0, l_lo + l_step * (int)blockIdx.y) + m;
     const int j0 = m % b.SX - 2, j1 = j0 == b.nx + 3 ? -2 : j0 + 1;
     const bool faces = lane >= 1 && lane <= 29;
     const bool ok0 = faces && m < cells && j0 >= 0 && j0 <= b.nx;
     const bool ok1 = faces && m + 1 < cells && j1 >= 0 && j1 <= b.nx;
     const AxisTabs A = T.ax[0];
     const R* src[7] = {pr.w[0], pr.w[1], pr.w[2], pr.w[3], pr.w[4], pr.bc[1], pr.bc[2]};
+    const auto W0 = xpair_weights<RECON, R>(A, j0, b.nx), W1 = xpair_weights<RECON, R>(A, j1, b.nx);
 #pragma unroll
     for (int v = 0; v < 7; ++v) {
         const Pair<R> x = ld_pair<VEC>(src[v], g);
         const R xm = __shfl_up_sync(FULL, x.b, 1), xp = __shfl_down_sync(FULL, x.a, 1);
         R vm0, vp0, vm1, vp1;
-        if (RECON == 4) {
-            const R d0 = ppm_slope(xm, x.a, x.b, (R)A.s0[j0], (R)A.s1[j0]);
-            const R d1 = ppm_slope(x.a, x.b, xp, (R)A.s0[j1], (R)A.s1[j1]);
+        if constexpr (RECON == 4) {
+            const R d0 = W0.slope(xm, x.a, x.b), d1 = W1.slope(x.a, x.b, xp);
             const R d2 = __shfl_down_sync(FULL, d0, 1);
-            const R V0 = ppm_face(x.a, x.b, d0, d1, (R)A.a0[j0], (R)A.a1[j0], (R)A.a2[j0], (R)A.a3[j0]);
-            const R V1 = ppm_face(x.b, xp, d1, d2, (R)A.a0[j1], (R)A.a1[j1], (R)A.a2[j1], (R)A.a3[j1]);
+            const R V0 = W0.face(x.a, x.b, d0, d1), V1 = W1.face(x.b, xp, d1, d2);
             const R Vm = __shfl_up_sync(FULL, V1, 1);
             ppm_fix(x.a, Vm, V0, vm0, vp0);
             ppm_fix(x.b, V0, V1, vm1, vp1);
         } else {
-            const R s0 = tvd_slope(xm, x.a, x.b, (R)A.tcf[j0], (R)A.tcb[j0]);
-            const R s1 = tvd_slope(x.a, x.b, xp, (R)A.tcf[j1], (R)A.tcb[j1]);
+            const R s0 = W0.slope(xm, x.a, x.b), s1 = W1.slope(x.a, x.b, xp);
             vm0 = x.a - R(0.5) * s0;
             vp0 = x.a + R(0.5) * s0;
             vm1 = x.b - R(0.5) * s1;

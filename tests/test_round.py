@@ -40,6 +40,22 @@ __global__ void k(long n, const double* a, const double* b, double* q, double* r
     const double s = rsqrt_seed(b[i]);
     es[i] = fma(-(b[i] * s), s, 1.0);
 }
+__global__ void kf(long n, const float* x, float* q, float* r) {
+    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    q[i] = recip_f(x[i]);
+    r[i] = root_f(x[i]);
+}
+extern "C" int runf(long n, const float* x, float* out) {
+    float *dx, *d;
+    const size_t bytes = n * sizeof(float);
+    if (cudaMalloc(&dx, bytes) || cudaMalloc(&d, 2 * bytes)) return 1;
+    cudaMemcpy(dx, x, bytes, cudaMemcpyHostToDevice);
+    kf<<<(unsigned)((n + 255) / 256), 256>>>(n, dx, d, d + n);
+    const int rc = cudaMemcpy(out, d, 2 * bytes, cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(dx), cudaFree(d);
+    return rc;
+}
 extern "C" int run(long n, const double* a, const double* b, double* out) {
     double *da, *db, *d;
     const size_t bytes = n * sizeof(double);
@@ -144,13 +160,31 @@ def test_quotients_and_roots_cpu(tmp_path):
         assert _same(r[keep], np.sqrt(b)[keep]), err
 
 
-@pytest.mark.gpu
-def test_quotients_and_roots_gpu(tmp_path):
-    src, so = tmp_path / "r.cu", tmp_path / "r.so"
+@pytest.fixture(scope="module")
+def gpu_lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("round")
+    src, so = d / "r.cu", d / "r.so"
     src.write_text(GPU_SRC)
     subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "--fmad=false",
                     "-shared", "-Xcompiler", "-fPIC", "-o", str(so), str(src)], check=True)
-    lib = ctypes.CDLL(str(so))
+    return ctypes.CDLL(str(so))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("exponent", [-100, -61, -38, -1, 0, 1, 44, 60, 99])
+def test_fp32_reciprocals_and_roots_gpu(gpu_lib, exponent):
+    """every significand at one exponent (with its neighbour: both parities)"""
+    x = (np.arange(2 ** 23, dtype=np.uint32) + np.uint32((exponent + 127) << 23)).view(np.float32)
+    out = np.empty((2, len(x)), dtype=np.float32)
+    fp = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_float))  # noqa: E731
+    assert gpu_lib.runf(ctypes.c_long(len(x)), fp(x), fp(out)) == 0
+    assert np.array_equal(out[0].view(np.int32), (np.float32(1.0) / x).view(np.int32))
+    assert np.array_equal(out[1].view(np.int32), np.sqrt(x).view(np.int32))
+
+
+@pytest.mark.gpu
+def test_quotients_and_roots_gpu(gpu_lib):
+    lib = gpu_lib
     a, b, _ = operands(4_000_000, True)
     a = np.concatenate([a, [0.0, -0.0, 0.0, -0.0]])  # zeros keep their sign
     b = np.concatenate([b, [1.0, 3.0, 0.7, 2.0 ** -200]])
