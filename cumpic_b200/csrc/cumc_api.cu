@@ -113,6 +113,9 @@ struct cumc_ctx {
     size_t adj_slab_bytes = 0;
     int next_stage = 1;    // cumc_rk_stage: the stage due next
     int part1_stage = 0;   // cumc_rk_stage_part: the stage whose part 1 ran and whose part 2 is due
+    cudaStream_t side[2]{};      // the y and z sweeps beside the x sweep (beside())
+    cudaEvent_t ev_fork = nullptr, ev_join[2]{};
+    bool fork = false;     // the stage's three sweeps run side by side (inside a step's graph only)
     bool fuse_dt = false;  // stage 3 also forms the next step's CFL dt (cumc_advance, cumc_rungekutta)
     bool dt_valid = false; // dtmin holds the CFL dt of the current state (set by cumc_rungekutta only)
     int bf_set = 0;        // U[bf_set] holds the current face fields (the last stage's output)
@@ -498,7 +501,38 @@ void mx_post(void* u, int cls) {
     ++c->launches;
     if (c->prof_on && cls >= 0) cudaEventRecord(c->prof.back().b, c->stream);
 }
-Launcher mx_launcher(cumc_ctx* c) { return Launcher{c->stream, mx_pre, mx_post, c}; }
+Launcher mx_launcher(cumc_ctx* c) {
+    return Launcher{c->stream, mx_pre, mx_post, c, c->fork, {c->side[0], c->side[1]}, c->ev_fork,
+                    {c->ev_join[0], c->ev_join[1]}};
+}
+
+// The three sweeps of a stage read the same primitives and write their own
+// fluxes. Inside a step's graph the y and z sweeps are put on side branches: on
+// small boxes each of the three is one wave of latency-bound blocks, and on
+// larger ones a sweep's last blocks leave room for the next one's first: a step
+// of the 512x4x4 tube 0.128 -> 0.105 ms, 64^3 0.363 -> 0.338, the 192x128x64
+// torus 1.84 -> 1.75, 256^3 2 % less.
+// beside() issues `work` on side branch n, join() makes the context's stream wait
+// for the branches; elsewhere (per-kernel timing, single launches) the work
+// goes on the context's stream in order.
+template <typename F>
+void beside(cumc_ctx* c, int n, F&& work) {
+    if (!c->fork) {
+        work();
+        return;
+    }
+    if (n == 0) cudaEventRecord(c->ev_fork, c->stream);
+    const cudaStream_t main = c->stream;
+    c->stream = c->side[n];
+    cudaStreamWaitEvent(c->stream, c->ev_fork, 0);
+    work();
+    cudaEventRecord(c->ev_join[n], c->stream);
+    c->stream = main;
+}
+void join(cumc_ctx* c) {
+    if (!c->fork) return;
+    for (cudaEvent_t e : c->ev_join) cudaStreamWaitEvent(c->stream, e, 0);
+}
 
 // One SPATIAL + combine + conversions + boundary (solver/rungekutta.f90:38-66).
 // stage 0: SPATIAL only, l_rk stored in c->L.
@@ -702,11 +736,13 @@ void run_stage(cumc_ctx* c, const Box& b, int stage, int part = 0) {
     if (split && part == 2) {  // the rest: the x and y sweeps of the ghost planes 0 and nz+1 first
         sweep<0>(c, b, pr, 0, 2, b.nz + 1);
         sweep<1>(c, b, pr, 0, 2, b.nz + 1);
+        sweep<2>(c, b, pr);
     } else {
+        beside(c, 0, [&] { sweep<1>(c, b, pr); });
+        beside(c, 1, [&] { sweep<2>(c, b, pr); });
         sweep<0>(c, b, pr);
-        sweep<1>(c, b, pr);
+        join(c);
     }
-    sweep<2>(c, b, pr);
     FaceFlux ff[3];
     for (int d = 0; d < 3; ++d)
         for (int q = 0; q < 7; ++q) ff[d].f[q] = c->F[d][q];
@@ -775,7 +811,9 @@ int rk_step_host(cumc_ctx* c) {
         cudaGraph_t g;
         const long long before = c->launches;
         CUMC_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        c->fork = true;
         rk_step_dt(c, c->box);
+        c->fork = false;
         c->rk_launches = c->launches - before;
         c->launches = before;
         CUMC_CHECK(cudaStreamEndCapture(c->stream, &g));
@@ -1123,10 +1161,18 @@ int cumc_init(const cumc_config* cfg, cumc_ctx** out) {
         cuda_fail(c, e, "cudaFuncSetAttribute(mixed sweep smem)");
         return fail_init(CUMC_ERR_CUDA);
     }
-    if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) {
-        cuda_fail(c, e, "cudaStreamCreate");
-        return fail_init(CUMC_ERR_CUDA);
-    }
+    cudaStream_t* streams[3] = {&c->stream, &c->side[0], &c->side[1]};
+    for (cudaStream_t* st : streams)
+        if ((e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking)) != cudaSuccess) {
+            cuda_fail(c, e, "cudaStreamCreate");
+            return fail_init(CUMC_ERR_CUDA);
+        }
+    cudaEvent_t* events[3] = {&c->ev_fork, &c->ev_join[0], &c->ev_join[1]};
+    for (cudaEvent_t* ev : events)
+        if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) {
+            cuda_fail(c, e, "cudaEventCreate");
+            return fail_init(CUMC_ERR_CUDA);
+        }
 
     // tables
     const int st[3] = {b.nx + 7, b.ny + 7, b.nz + 7};
@@ -1270,7 +1316,10 @@ int cumc_free(cumc_ctx* c) {
     if (c->snap_taken) cudaEventDestroy(c->snap_taken);
     if (c->snap_done) cudaEventDestroy(c->snap_done);
     if (c->host_pinned) cudaFreeHost(c->host_pinned);
-    if (c->stream) cudaStreamDestroy(c->stream);
+    for (cudaEvent_t ev : {c->ev_fork, c->ev_join[0], c->ev_join[1]})
+        if (ev) cudaEventDestroy(ev);
+    for (cudaStream_t st : {c->side[0], c->side[1], c->stream})
+        if (st) cudaStreamDestroy(st);
     delete c;
     return CUMC_OK;
 }
@@ -1539,8 +1588,10 @@ int cumc_advance(cumc_ctx* c, int nsteps, double t_end, double* t_inout, int* st
             cudaGraph_t g;
             CUMC_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             const long long before = c->launches;
-                loop_step(c, t_end);
-                const long long per_step = c->launches - before;
+            c->fork = true;
+            loop_step(c, t_end);
+            c->fork = false;
+            const long long per_step = c->launches - before;
             c->launches = before;
             CUMC_CHECK(cudaStreamEndCapture(c->stream, &g));
             cudaError_t e = cudaGraphInstantiate(&c->graph_exec, g, 0);

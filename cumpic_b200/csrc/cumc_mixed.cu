@@ -841,9 +841,22 @@ void mixed_stage(const Launcher& L, const Box& b, const Tabs& T, const MixedBufs
     for (int q = 0; q < 5; ++q) pr.w[q] = m.w[q];
     for (int q = 0; q < 3; ++q) { pr.bc[q] = m.bc[q]; pr.bf[q] = m.bf[q]; }
     const float ggas = (float)p.ggas;
+    Launcher branch[2] = {L, L};
+    if (L.fork) {
+        cudaEventRecord(L.ev_fork, L.stream);
+        for (int n = 0; n < 2; ++n) {
+            branch[n].stream = L.side[n];
+            cudaStreamWaitEvent(L.side[n], L.ev_fork, 0);
+        }
+    }
+    sweep_mx<1>(branch[0], b, T, pr, ggas, m, p.recon, p.sm_count, p.hll_fp32 != 0);
+    sweep_mx<2>(branch[1], b, T, pr, ggas, m, p.recon, p.sm_count, p.hll_fp32 != 0);
     sweep_mx<0>(L, b, T, pr, ggas, m, p.recon, p.sm_count, p.hll_fp32 != 0);
-    sweep_mx<1>(L, b, T, pr, ggas, m, p.recon, p.sm_count, p.hll_fp32 != 0);
-    sweep_mx<2>(L, b, T, pr, ggas, m, p.recon, p.sm_count, p.hll_fp32 != 0);
+    if (L.fork)
+        for (int n = 0; n < 2; ++n) {
+            cudaEventRecord(L.ev_join[n], L.side[n]);
+            cudaStreamWaitEvent(L.stream, L.ev_join[n], 0);
+        }
     FaceFluxT<float> ff[3];
     for (int d = 0; d < 3; ++d)
         for (int q = 0; q < 7; ++q) ff[d].f[q] = m.F[d][q];

@@ -52,6 +52,11 @@ struct Launcher {
     void (*pre)(void* user, int cls);
     void (*post)(void* user, int cls);
     void* user;
+    // fork: the y and z sweeps on branches of their own beside the x sweep
+    // (inside a step's graph; see beside() in cumc_api.cu)
+    bool fork = false;
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
 };
 
 cudaError_t mixed_attributes();
