@@ -115,6 +115,7 @@ struct cumc_ctx {
     int part1_stage = 0;   // cumc_rk_stage_part: the stage whose part 1 ran and whose part 2 is due
     cudaStream_t side[2]{};      // the y and z sweeps beside the x sweep (beside())
     cudaEvent_t ev_fork = nullptr, ev_join[2]{};
+    bool whole_step = false;  // inside rk_step: no caller sees the state between the stages
     bool fork = false;     // the stage's three sweeps run side by side (inside a step's graph only)
     bool fuse_dt = false;  // stage 3 also forms the next step's CFL dt (cumc_advance, cumc_rungekutta)
     bool dt_valid = false; // dtmin holds the CFL dt of the current state (set by cumc_rungekutta only)
@@ -765,6 +766,7 @@ void run_stage(cumc_ctx* c, const Box& b, int stage, int part = 0) {
     a.dt = c->scal;
     for (int q = 0; q < 3; ++q) a.ecorn[q] = c->E[q];
     a.geom_repeat = c->cfg.geom_source_repeat;
+    a.lean = c->whole_step;
     a.rho_floor = c->cfg.rho_floor;
     a.r_sh = c->cfg.r_sh;
     // adjoint recomputation: the combine's output of this stage, on (0:n)^3.
@@ -786,9 +788,11 @@ void run_stage(cumc_ctx* c, const Box& b, int stage, int part = 0) {
 }
 
 void rk_step(cumc_ctx* c, const Box& b) {
+    c->whole_step = true;
     run_stage(c, b, 1);
     run_stage(c, b, 2);
     run_stage(c, b, 3);
+    c->whole_step = false;
 }
 
 // rk_step with the next step's dt formed at stage 3
