@@ -11,7 +11,7 @@
 // plane's edges average, then the edge EMFs of the tile and of the halo row
 // and column its CT reads (Ez at j-1 and k-1; Ey at j-1; Ex at k-1), and
 // keeps the x and y edge EMFs of the previous plane (the l-1 edges of CT).
-// Each cell EMF is formed once per plane, each edge EMF at most 1.2 times.
+// Each cell EMF is formed at most 1.6 times, each edge EMF 1.3 times.
 // Edges with an index of -1 are zero, as the never-written entries of the
 // edge arrays are for k_ct. Every value is the same expression, in the same
 // order, as in k_emf and k_ct, so the result is bit for bit theirs.
@@ -20,12 +20,17 @@
 
 namespace cumc {
 
+// Face triples of a tile. Smaller tiles form more halo edges and cells (1.29
+// and 1.59 a triple at 32 x 4, 1.16 and 1.33 at 32 x 8), but a block waits at
+// its barriers for fewer warps. 32 x 8 -> 32 x 4: 0.717 -> 0.675 ms a stage at
+// 256^3, 0.115 -> 0.091 on the 192x128x64 torus, 0.027 -> 0.023 at 64^3; 32 x 2
+// takes 0.76, 0.098 and 0.025.
 #ifndef CUMC_EC_TY
-#define CUMC_EC_TY 8
+#define CUMC_EC_TY 4
 #endif
-constexpr int EC_TX = 32, EC_TY = CUMC_EC_TY;  // face triples of a tile
-constexpr int EC_CX = EC_TX + 2, EC_CY = EC_TY + 2;  // cells j0-1..j0+32, k0-1..k0+8
-constexpr int EC_EX = EC_TX + 1, EC_EY = EC_TY + 1;  // edges j0-1..j0+31, k0-1..k0+7
+constexpr int EC_TX = 32, EC_TY = CUMC_EC_TY;
+constexpr int EC_CX = EC_TX + 2, EC_CY = EC_TY + 2;  // cells j0-1..j0+32, k0-1..k0+4
+constexpr int EC_EX = EC_TX + 1, EC_EY = EC_TY + 1;  // edges j0-1..j0+31, k0-1..k0+3
 
 // shared memory of a tile; R is the EMFs' type (double, or float in the
 // mixed form)
@@ -189,7 +194,7 @@ __device__ __forceinline__ void ct_curl(const CTf& g, double Ex, double Ex_lm, d
 // its edges overwrite slots that CT reads, which every thread has finished
 // before it reaches the next plane's first barrier.
 #ifndef CUMC_EC_MINB
-#define CUMC_EC_MINB 4
+#define CUMC_EC_MINB 8
 #endif
 template <int COORD, int STAGE>
 __global__ void __launch_bounds__(EC_TX * EC_TY, CUMC_EC_MINB) k_emf_ct(Box b, Tabs T, Prim pr, FaceFlux fx,

@@ -251,7 +251,7 @@ struct CtMx {
 };
 
 #ifndef CUMC_ECMX_MINB
-#define CUMC_ECMX_MINB 6
+#define CUMC_ECMX_MINB 10
 #endif
 template <int COORD, int STAGE>
 __global__ void __launch_bounds__(EC_TX * EC_TY, CUMC_ECMX_MINB) k_emf_ct_mx(Box b, Tabs T, PrimT<float> pr, FaceFluxT<float> fx,
