@@ -22,9 +22,8 @@ COMMON = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcom
 FP64_FLAGS = ["--fmad=false"]
 # mixed path: FMA contraction; IEEE-rounded FP32 division and square root (the
 # approximate forms raise the density error at t_end from 1.06e-5 to 1.5e-5 on
-# Orszag-Tang 256^3); the column walker compiled for 10 blocks a SM (96
-# registers) instead of the FP64 unit's 8.
-MIXED_FLAGS = ["--fmad=true", "-prec-div=true", "-prec-sqrt=true", "-DCUMC_WALK_MINB=10"]
+# Orszag-Tang 256^3).
+MIXED_FLAGS = ["--fmad=true", "-prec-div=true", "-prec-sqrt=true"]
 UNITS = {"cumc_api.cu": FP64_FLAGS, "cumc_mixed.cu": MIXED_FLAGS, "cumc_static.cu": FP64_FLAGS}
 NVCC_FLAGS = COMMON + FP64_FLAGS  # flags of the FP64 unit (kept for tools that print them)
 

@@ -283,7 +283,7 @@ void sweep(cumc_ctx* c, const Box& b, const Prim& pr, int l_lo = 0, int l_cnt = 
         const int cls = CUMC_K_SWEEP_X + DIR;
         if (mode == 4 || mode == 0 || mode == 7) {
             const bool ppm = c->recon == CUMC_PPMC;
-            const size_t sm = walk_smem<double>(DIR, ppm);
+            const size_t sm = walk_smem<double>(DIR, ppm, seg);
             if (c->fast)
                 launch_grid(c, cls, grid, WK_THREADS, sm,
                             ppm ? k_sweep_walk_sm<DIR, 4, double, false, true> : k_sweep_walk_sm<DIR, 1, double, false, true>,
@@ -1812,7 +1812,7 @@ void adj_sweeps(cumc_ctx* c, const Box& b, const Prim& pr, const AdjStage& st, c
         int nseg;
         const int seg = walk_segment_for<D>(b, WalkGeom<D>::ncols(b), c->sm_count, &nseg);
         const dim3 grid((unsigned)((WalkGeom<D>::ncols(b) + WK_THREADS - 1) / WK_THREADS), (unsigned)nseg);
-        launch_grid(c, -1, grid, WK_THREADS, walk_smem<double>(D, RECON == 4), k_sweep_walk_sm<D, RECON, double, true>, b, c->tabs,
+        launch_grid(c, -1, grid, WK_THREADS, walk_smem<double>(D, RECON == 4, seg), k_sweep_walk_sm<D, RECON, double, true>, b, c->tabs,
                     pr, c->ggas, sl, seg, sr, 0, -1, 1);
     };
     // x: pass A per face, pass B one lane per cell and field

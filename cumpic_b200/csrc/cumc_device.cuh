@@ -151,6 +151,12 @@ struct CellWeights {  // PPM: slope weights of cell c, interface weights of the 
     R s0, s1, a0, a1, a2, a3;
     __device__ __forceinline__ CellWeights(const AxisTabs& A, int cs, int cf)
         : s0((R)A.s0[cs]), s1((R)A.s1[cs]), a0((R)A.a0[cf]), a1((R)A.a1[cf]), a2((R)A.a2[cf]), a3((R)A.a3[cf]) {}
+    static constexpr int N = 6;  // stored weights a face, in the order of the constructor below
+    __device__ __forceinline__ CellWeights(const R* t, int n)
+        : s0(t[0]), s1(t[n]), a0(t[2 * n]), a1(t[3 * n]), a2(t[4 * n]), a3(t[5 * n]) {}
+    __device__ __forceinline__ void store(R* t, int n) const {
+        t[0] = s0, t[n] = s1, t[2 * n] = a0, t[3 * n] = a1, t[4 * n] = a2, t[5 * n] = a3;
+    }
     __device__ __forceinline__ R slope(R vm, R vc, R vp) const { return ppm_slope(vm, vc, vp, s0, s1); }
     __device__ __forceinline__ R face(R vc, R vp, R dmc, R dmp) const {
         return ppm_face(vc, vp, dmc, dmp, a0, a1, a2, a3);
@@ -159,7 +165,10 @@ struct CellWeights {  // PPM: slope weights of cell c, interface weights of the 
 template <typename R>
 struct CellWeights<1, R> {  // TVD
     R cf, cb;
+    static constexpr int N = 2;
     __device__ __forceinline__ CellWeights(const AxisTabs& A, int c) : cf((R)A.tcf[c]), cb((R)A.tcb[c]) {}
+    __device__ __forceinline__ CellWeights(const R* t, int n) : cf(t[0]), cb(t[n]) {}
+    __device__ __forceinline__ void store(R* t, int n) const { t[0] = cf, t[n] = cb; }
     __device__ __forceinline__ R slope(R vm, R vc, R vp) const { return tvd_slope(vm, vc, vp, cf, cb); }
 };
 // TVD in FP64: the quotients by cf and cb share their reciprocals over the
@@ -169,6 +178,7 @@ struct CellWeights<1, double> {
     double cf, cb;
     Recip rf, rb;
     bool ok;
+    static constexpr int N = 2;
     __device__ __forceinline__ CellWeights(const AxisTabs& A, int c) : cf(A.tcf[c]), cb(A.tcb[c]) {
         ok = range_max(cf, range_max(cb, 0u)) < RANGE_SPAN;
         rf = recip_of(cf);

@@ -669,7 +669,7 @@ void sweep_mx(const Launcher& L, const Box& b, const Tabs& T, const PrimT<float>
         int nseg;
         const int seg = walk_segment_for<D>(b, WalkGeom<D>::ncols(b), sm_count, &nseg);
         const dim3 grid((unsigned)((WalkGeom<D>::ncols(b) + WK_THREADS - 1) / WK_THREADS), (unsigned)nseg);
-        const size_t sm = walk_smem<float>(D, ppm);
+        const size_t sm = walk_smem<float>(D, ppm, seg);
         if (fp32)
             run(L, DIR, grid, WK_THREADS, sm,
                 ppm ? k_sweep_walk_sm<D, 4, float, false, true> : k_sweep_walk_sm<D, 1, float, false, true>, b, T, pr,

@@ -63,17 +63,14 @@ struct WalkGeom {
 // 8 while the grid gave fewer than 32 warps a SM: 64^3 0.036 -> 0.029 ms a
 // walk, the 90x26x75 torus 0.029 -> 0.023, a 512x4x4 tube 0.021 -> 0.013; 256^3
 // unchanged (0.90).
-#ifndef CUMC_WALK_RES
-#define CUMC_WALK_RES 10
-#endif
-constexpr int WK_RESIDENT = CUMC_WALK_RES;
+constexpr int WK_RESIDENT = 10, WK_SEG_MAX = 64;  // (64 faces: 3 KB of weights a block)
 template <int DIR>
 inline int walk_segment_for(const Box& b, long long ncols, int sm_count, int* nseg) {
     const int faces = WalkGeom<DIR>::nd(b) + 1;
     const long long blocks = (ncols + WK_THREADS - 1) / WK_THREADS, slots = (long long)sm_count * WK_RESIDENT;
     long long best = -1;
     int best_seg = faces;
-    for (int n = 1; n <= faces; ++n) {
+    for (int n = (faces + WK_SEG_MAX - 1) / WK_SEG_MAX; n <= faces; ++n) {
         const int seg = (faces + n - 1) / n;
         const long long rounds = (blocks * ((faces + seg - 1) / seg) + slots - 1) / slots;
         const long long cost = rounds * (2 * seg + 3);
@@ -350,9 +347,17 @@ struct WalkSlots {
     static constexpr int RING = RECON == 4 ? 2 : 3, D1 = RING, VF = RING + 1, VP = RECON == 4 ? RING + 2 : RING,
                          COUNT = VP + 1;
 };
+// The mixed form's walkers also keep the weights of the segment's faces, rounded
+// to FP32 once a block: 0.541 -> 0.527 (y) and 0.520 ms (z) at 256^3. In FP64 the
+// weights come from global memory at every face, the same 0.90 ms.
 template <typename R>
-inline size_t walk_smem(int dir, bool ppm) {
-    return (size_t)(ppm ? WalkSlots<4>::COUNT : WalkSlots<1>::COUNT) * WK_FIELDS * WK_THREADS * sizeof(R) +
+constexpr bool WALK_TAB = sizeof(R) == 4;
+// the window, then the weights (CellWeights::store), then the x staging
+template <typename R>
+inline size_t walk_smem(int dir, bool ppm, int seg) {
+    const int w = !WALK_TAB<R> ? 0 : ppm ? CellWeights<4, R>::N : CellWeights<1, R>::N;
+    return ((size_t)(ppm ? WalkSlots<4>::COUNT : WalkSlots<1>::COUNT) * WK_FIELDS * WK_THREADS + (size_t)w * seg) *
+               sizeof(R) +
            (dir == 0 ? xstage_smem<R>() : 0);
 }
 constexpr int WK_SLOTS = 6;  // slots of the fused walkers (cumc_fused.cuh): a ring of three, slope, interface, vp_out
@@ -375,7 +380,10 @@ __global__ void __launch_bounds__(WK_THREADS, CUMC_WALK_MINB) k_sweep_walk_sm(Bo
     const int s = C.s, f0 = C.f0;
     XStage<R> X;
     using W = WalkSlots<RECON>;
-    if (DIR == 0) X.init(b, pr, reinterpret_cast<R*>(wk_raw) + W::COUNT * WK_FIELDS * WK_THREADS);
+    R* const tab = reinterpret_cast<R*>(wk_raw) + W::COUNT * WK_FIELDS * WK_THREADS;
+    if constexpr (WALK_TAB<R>)
+        for (int n = threadIdx.x; n < C.f1 - f0; n += WK_THREADS) walk_weights<RECON, R>(A, f0 + n).store(tab + n, seg);
+    if (DIR == 0) X.init(b, pr, tab + (WALK_TAB<R> ? CellWeights<RECON, R>::N * seg : 0));
 
     R nxt[WK_FIELDS];
     // ring positions of v(f), v(f+1), v(f+2) for f = f0 (a ring of two has no v(f))
@@ -397,13 +405,22 @@ __global__ void __launch_bounds__(WK_THREADS, CUMC_WALK_MINB) k_sweep_walk_sm(Bo
         at(W::VP, v) = vpf;
         nxt[v] = q[(f0 + 3) * s];
     }
+    // the mixed form fetches the normal field a face ahead too (its faces are short
+    // enough to wait for it: z 0.519 -> 0.484 ms); FP64 has no register for it
+    constexpr bool AHEAD = DIR > 0 && sizeof(R) == 4;
+    R bn_next = AHEAD ? C.bn[f0 * s] : R(0);
+    if constexpr (WALK_TAB<R>) __syncthreads();
 
     for (int f = f0; f < C.f1; ++f) {
         R wl[8], wr[8];
         const int j = (f - f0) & (XS_CELLS - 1);
         if (DIR == 0 && j == 0) walk_chunk(C, f, X, out);
-        const R bn = DIR == 0 ? X.get(WK_FIELDS, j) : C.bn[f * s];
-        const auto cw = walk_weights<RECON, R>(A, f);
+        const R bn = DIR == 0 ? X.get(WK_FIELDS, j) : AHEAD ? bn_next : C.bn[f * s];
+        auto weights = [&] {
+            if constexpr (WALK_TAB<R>) return CellWeights<RECON, R>(tab + (f - f0), seg);
+            else return walk_weights<RECON, R>(A, f);
+        };
+        const CellWeights<RECON, R> cw = weights();
 #pragma unroll
         for (int v = 0; v < WK_FIELDS; ++v) {
             const R x = nxt[v];
@@ -432,6 +449,7 @@ __global__ void __launch_bounds__(WK_THREADS, CUMC_WALK_MINB) k_sweep_walk_sm(Bo
         if (f + 1 < C.f1) {
 #pragma unroll
             for (int v = 0; v < WK_FIELDS; ++v) nxt[v] = DIR == 0 ? X.get(v, j) : C.src[v][(f + 4) * s];
+            if (AHEAD) bn_next = C.bn[(f + 1) * s];
         }
         if (STATES) {
             if (C.active) {
