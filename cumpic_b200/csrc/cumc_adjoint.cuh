@@ -1044,7 +1044,7 @@ __global__ void __launch_bounds__(256) k_adj_prims(Box b, Arr8 src, UtopArgs a) 
 template <int MODEL, bool FROM_CONS>
 __global__ void __launch_bounds__(256) k_adj_utop(Box b, Arr8 u, Arr8 w0, const double* eps0, Arr8 lu,
                                                   AdjPrim o, double ggas, Arr8 mu, Arr3 lb, double alpha,
-                                                  double beta, Arr8 lam0) {
+                                                  double beta, Arr8 lam0, bool first) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1056,6 +1056,7 @@ __global__ void __launch_bounds__(256) k_adj_utop(Box b, Arr8 u, Arr8 w0, const 
         for (int q = 0; q < 5; ++q) {
             mu.a[q][i] = 0.0;
             if (beta != 0.0) lu.a[q][i] = 0.0;
+            if (FROM_CONS && first) lam0.a[q][i] = 0.0;
         }
 #pragma unroll
         for (int q = 0; q < 3; ++q) lb.a[q][i] = 0.0;
@@ -1132,9 +1133,18 @@ __global__ void __launch_bounds__(256) k_adj_utop(Box b, Arr8 u, Arr8 w0, const 
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
             const double m = mu.a[q][i];
-            lam0.a[q][i] += alpha * m;
+            lam0.a[q][i] = first ? alpha * m : lam0.a[q][i] + alpha * m;
             if (beta != 0.0) lu.a[q][i] = beta * m;
         }
+    }
+    // the primitive adjoints are spent (the boundary's transpose has cleared the
+    // ghosts'): cleared here for the next stage to add to
+    if (FROM_CONS) {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) o.w[q][i] = 0.0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) o.bc[q][i] = 0.0;
+        o.eps[i] = 0.0;
     }
 }
 
@@ -1142,7 +1152,7 @@ __global__ void __launch_bounds__(256) k_adj_utop(Box b, Arr8 u, Arr8 w0, const 
 // values plus half the adjoints of the two active cells whose bcell average
 // reads the face (solver/fromrvetou.f90:97-107); zero on every other entry
 __global__ void __launch_bounds__(256) k_adj_bface(Box b, Arr3 lbf, Arr3 lb, Arr3 out, double alpha, double beta,
-                                                   Arr3 lam0) {
+                                                   Arr3 lam0, bool first) {
     const int n0 = b.nx + 1, n1 = b.ny + 1, n2 = b.nz + 1;
     const long long total = (long long)n0 * n1 * n2;
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1168,7 +1178,7 @@ __global__ void __launch_bounds__(256) k_adj_bface(Box b, Arr3 lbf, Arr3 lb, Arr
         out.a[d][i] = v;
         // combine^T of the field part (lbf, read above by this thread only,
         // becomes the adjoint of the previous stage's face field)
-        if (alpha != 0.0) lam0.a[d][i] += alpha * v;
+        if (alpha != 0.0) lam0.a[d][i] = first ? alpha * v : lam0.a[d][i] + alpha * v;
         if (beta != 0.0) lbf.a[d][i] = beta * v;
     }
 }

@@ -1854,12 +1854,14 @@ void adj_spatial(cumc_ctx* c, const Box& b, const Prim& pr, const AdjStage& st, 
 
 template <bool FROM_CONS>
 void adj_utop(cumc_ctx* c, const Box& b, Arr8 u, Arr8 w0, const double* eps0, Arr8 lu, const AdjPrim& lp, Arr8 mu,
-              Arr3 lb, double alpha = 0.0, double beta = 0.0, Arr8 lam0 = Arr8{}) {
+              Arr3 lb, double alpha = 0.0, double beta = 0.0, Arr8 lam0 = Arr8{}, bool first = false) {
     const long long n = (long long)(b.nx + 1) * (b.ny + 1) * (b.nz + 1);
     if (c->model == CUMC_MODEL_RIEMANN)
-        launch(c, -1, n, 256, k_adj_utop<1, FROM_CONS>, b, u, w0, eps0, lu, lp, c->ggas, mu, lb, alpha, beta, lam0);
+        launch(c, -1, n, 256, k_adj_utop<1, FROM_CONS>, b, u, w0, eps0, lu, lp, c->ggas, mu, lb, alpha, beta, lam0,
+               first);
     else
-        launch(c, -1, n, 256, k_adj_utop<0, FROM_CONS>, b, u, w0, eps0, lu, lp, c->ggas, mu, lb, alpha, beta, lam0);
+        launch(c, -1, n, 256, k_adj_utop<0, FROM_CONS>, b, u, w0, eps0, lu, lp, c->ggas, mu, lb, alpha, beta, lam0,
+               first);
 }
 
 int adjoint_run(cumc_ctx* c, int N, int K, int obj, const double* weights, const double* dt_in, double* dt_out,
@@ -1971,7 +1973,7 @@ int adjoint_run(cumc_ctx* c, int N, int K, int obj, const double* weights, const
 
     // ---- objective and seed --------------------------------------------------
     double** lamCur = lamA;  // adjoint of the state at the current stage boundary
-    double** lamU0 = lamB;   // adjoint of the step's starting state (accumulated)
+    double** lamU0 = lamB;   // adjoint of the step's starting state (set at stage 3, then accumulated)
     if (obj == CUMC_OBJ_LINEAR) {
         if ((rc = put_soa(c, weights, 8, lamCur)) != CUMC_OK) return rc;
         launch(c, -1, (long long)NT, 256, k_adj_mask_live, b, arr8(lamCur));
@@ -2002,7 +2004,6 @@ int adjoint_run(cumc_ctx* c, int N, int K, int obj, const double* weights, const
         for (int n = a1 - 1; n >= a0; --n) {
             double* const* tp = &tape[(size_t)(n - a0) * 24];
             if (!have_next) adj_prims_from(c, b, tp + 16, P[pc]);
-            for (int q = 0; q < 8; ++q) zero(lamU0[q]);
             for (int s = 3; s >= 1; --s) {
                 StateSet& Pc = P[pc];
                 StateSet& Pp = P[1 - pc];
@@ -2013,10 +2014,9 @@ int adjoint_run(cumc_ctx* c, int N, int K, int obj, const double* weights, const
                 adj_boundary(c, b, bound_args(c, Pc.u, Pc.prim()), lp, lamCur + IBX);
                 // utop^T and the face-field gather, each with the combine^T of its part
                 adj_utop<true>(c, b, arr8(tp + (s - 1) * 8), arr8(Pc.w, 5), nullptr, arr8(lamCur), lp, arr8(mu), arr3(lb),
-                               alpha[s], beta[s], arr8(lamU0));
+                               alpha[s], beta[s], arr8(lamU0), s == 3);
                 launch(c, -1, (long long)(b.nx + 1) * (b.ny + 1) * (b.nz + 1), 256, k_adj_bface, b, arr3(lamCur + IBX),
-                       arr3(lb), arr3(mu + IBX), alpha[s], beta[s], arr3(lamU0 + IBX));
-                zero_lp();
+                       arr3(lb), arr3(mu + IBX), alpha[s], beta[s], arr3(lamU0 + IBX), s == 3);
                 // L^T at the stage's input
                 AdjStage st;
                 for (int q = 0; q < 8; ++q) st.mu[q] = mu[q];
@@ -2040,7 +2040,7 @@ int adjoint_run(cumc_ctx* c, int N, int K, int obj, const double* weights, const
     adj_boundary(c, b, bound_args(c, ck[0].u, ck[0].prim()), lp, lamCur + IBX);
     adj_utop<false>(c, b, arr8(ck[0].u), arr8(ck[0].w, 5), ck[0].eps, arr8(lamCur), lp, arr8(mu), arr3(lb));
     launch(c, -1, (long long)(b.nx + 1) * (b.ny + 1) * (b.nz + 1), 256, k_adj_bface, b, arr3(lamCur + IBX), arr3(lb),
-           arr3(mu + IBX), 0.0, 0.0, Arr3{});
+           arr3(mu + IBX), 0.0, 0.0, Arr3{}, false);
     if ((rc = sync_status(c)) != CUMC_OK) return rc;
     if (grad_prim) {
         const double* s[8] = {mu[0], mu[1], mu[2], mu[3], nullptr, mu[IBX], mu[IBY], mu[IBZ]};
