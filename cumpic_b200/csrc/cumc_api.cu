@@ -82,7 +82,7 @@ struct cumc_ctx {
     double graph_t_end = 0.0;
     long long graph_launches_per_step = 0;
     // sweep kernels (environment variable CUMC_SWEEP, for A/B timing; all
-    // give the same bits): 0 default (lane-per-cell x, shared-memory-window
+    // give the same bits): 0 default (two cells a lane along x, shared-memory-window
     // walker y/z), 1 "simple" (per-face everywhere), 2 "tile" (shared-memory tiles),
     // 3 "walkx" (register walker everywhere, x staged through shared memory),
     // 4 "walksm" (shared-memory-window walker everywhere), 5 "walkreg"

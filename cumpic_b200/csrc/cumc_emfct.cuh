@@ -32,6 +32,8 @@ constexpr int EC_TX = 32, EC_TY = CUMC_EC_TY;
 constexpr int EC_CX = EC_TX + 2, EC_CY = EC_TY + 2;  // cells j0-1..j0+32, k0-1..k0+4
 constexpr int EC_EX = EC_TX + 1, EC_EY = EC_TY + 1;  // edges j0-1..j0+31, k0-1..k0+3
 
+__host__ __device__ __forceinline__ int ec_tiles_x(const Box& b) { return (b.nx + 1 + EC_TX - 1) / EC_TX; }
+
 // shared memory of a tile; R is the EMFs' type (double, or float in the
 // mixed form)
 template <typename R>
@@ -205,8 +207,8 @@ __global__ void __launch_bounds__(EC_TX * EC_TY, CUMC_EC_MINB) k_emf_ct(Box b, T
     if (b.skip && *b.skip) return;
     constexpr int NE = EC_EX * EC_EY, NT = EC_TX * EC_TY;
     static_assert(NE > NT && NE <= 2 * NT, "two edges a thread at most");
-    const int j0 = blockIdx.x * EC_TX, k0 = blockIdx.y * EC_TY;
-    const int l0 = blockIdx.z * seg, l1 = min(l0 + seg, b.nz + 1);
+    const int tx = ec_tiles_x(b), j0 = (int)(blockIdx.x % tx) * EC_TX, k0 = (int)(blockIdx.x / tx) * EC_TY;
+    const int l0 = blockIdx.y * seg, l1 = min(l0 + seg, b.nz + 1);
     const int tj = threadIdx.x % EC_TX, tk = threadIdx.x / EC_TX;
     const int j = j0 + tj, k = k0 + tk;
     const bool mine = j <= b.nx && k <= b.ny;
@@ -263,19 +265,13 @@ __global__ void __launch_bounds__(EC_TX * EC_TY, CUMC_EC_MINB) k_emf_ct(Box b, T
 // halved down to 4 (and the plain quotients in the curl): 192x128x64 torus 0.129
 // -> 0.115 ms, the 90x26x75 one 0.029 -> 0.019, a 512x4x4 tube 0.020 -> 0.011,
 // 256^3 0.73 -> 0.72.
+// (x tile fastest, then y, in the grid's first dimension: the others end at
+// 65,535.)
 inline dim3 emf_ct_grid(const Box& b, long long slots, int* seg) {
-    const unsigned gx = (unsigned)((b.nx + 1 + EC_TX - 1) / EC_TX), gy = (unsigned)((b.ny + 1 + EC_TY - 1) / EC_TY);
-    const int planes = b.nz + 1;
-    long long best = -1;
-    for (int n = 1; n <= planes; ++n) {
-        const int s = (planes + n - 1) / n;
-        const long long rounds = ((long long)gx * gy * ((planes + s - 1) / s) + slots - 1) / slots;
-        if (best < 0 || rounds * (s + 1) < best) {
-            best = rounds * (s + 1);
-            *seg = s;
-        }
-    }
-    return dim3(gx, gy, (unsigned)((planes + *seg - 1) / *seg));
+    const long long tiles = (long long)ec_tiles_x(b) * ((b.ny + 1 + EC_TY - 1) / EC_TY);
+    int count;
+    *seg = segment_length(b.nz + 1, tiles, slots, 1, 1, b.nz + 1, &count);
+    return dim3((unsigned)tiles, (unsigned)count);
 }
 
 }  // namespace cumc

@@ -106,6 +106,30 @@ __global__ void __launch_bounds__(128) k_sweep(Box b, Tabs T, PrimT<R> pr, R gga
     for (int i = 0; i < 7; ++i) out.f[i][base] = fx[i];
 }
 
+// Length of the segments that `total` items along a direction are cut into, one
+// block each, for `blocks` such rows of segments: equal blocks run in rounds of
+// `slots` resident ones, a segment costs item * length + over, and the length is
+// taken that makes rounds x cost least (at most `most`). Only the most segments
+// that fit a number of rounds can be best, so those are tried.
+inline int segment_length(int total, long long blocks, long long slots, int item, int over, int most, int* count) {
+    const long long least = (total + most - 1) / most;
+    const long long first = (blocks * least + slots - 1) / slots;
+    long long best = -1;
+    int length = total;
+    for (long long r = first; r < first + 32; ++r) {
+        long long n = r * slots / blocks;
+        n = n < least ? least : n > total ? total : n;
+        const int len = (int)((total + n - 1) / n);
+        const long long rounds = (blocks * ((total + len - 1) / len) + slots - 1) / slots;
+        if (best < 0 || rounds * (item * len + over) < best) {
+            best = rounds * (item * len + over);
+            length = len;
+        }
+    }
+    *count = (total + length - 1) / length;
+    return length;
+}
+
 // ----------------------------------------------------------------------------
 // k_emf: edge EMFs on 0:n (solver/spatial.f90:190-203,268-281,346-359 then
 // solver/mhd.f90:95-125). ecorn is accumulated in the reference's sweep

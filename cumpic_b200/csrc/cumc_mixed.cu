@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(EC_TX * EC_TY, CUMC_ECMX_MINB) k_emf_ct_mx(Box
     EmfCtSmemT<float>& S = *reinterpret_cast<EmfCtSmemT<float>*>(ecm_raw);
     if (b.skip && *b.skip) return;
     constexpr int NE = EC_EX * EC_EY, NT = EC_TX * EC_TY;
-    const int j0 = blockIdx.x * EC_TX, k0 = blockIdx.y * EC_TY;
-    const int l0 = blockIdx.z * seg, l1 = min(l0 + seg, b.nz + 1);
+    const int tx = ec_tiles_x(b), j0 = (int)(blockIdx.x % tx) * EC_TX, k0 = (int)(blockIdx.x / tx) * EC_TY;
+    const int l0 = blockIdx.y * seg, l1 = min(l0 + seg, b.nz + 1);
     const int tj = threadIdx.x % EC_TX, tk = threadIdx.x / EC_TX;
     const int j = j0 + tj, k = k0 + tk;
     const bool mine = j <= b.nx && k <= b.ny;

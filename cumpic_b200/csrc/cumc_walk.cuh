@@ -30,8 +30,10 @@
 namespace cumc {
 
 constexpr int WK_THREADS = 64;
-// resident blocks per SM the walker and the x sweep are compiled for (the
-// register budget a thread gets); build-time tunables
+// resident blocks per SM the walker and the lane-per-cell x sweep are compiled
+// for (the register budget a thread gets); build-time tunables. The walker's 9
+// blocks of 64 get 96 registers, and 10 fit: 0.90 ms a stage at 256^3, FP64 pipe
+// 60 % busy; 7 and 8 blocks (128 registers) take 0.91, 11 and 12 (80) 0.93-0.94.
 #ifndef CUMC_WALK_MINB
 #define CUMC_WALK_MINB 9
 #endif
@@ -68,19 +70,7 @@ template <int DIR>
 inline int walk_segment_for(const Box& b, long long ncols, int sm_count, int* nseg) {
     const int faces = WalkGeom<DIR>::nd(b) + 1;
     const long long blocks = (ncols + WK_THREADS - 1) / WK_THREADS, slots = (long long)sm_count * WK_RESIDENT;
-    long long best = -1;
-    int best_seg = faces;
-    for (int n = (faces + WK_SEG_MAX - 1) / WK_SEG_MAX; n <= faces; ++n) {
-        const int seg = (faces + n - 1) / n;
-        const long long rounds = (blocks * ((faces + seg - 1) / seg) + slots - 1) / slots;
-        const long long cost = rounds * (2 * seg + 3);
-        if (best < 0 || cost < best) {
-            best = cost;
-            best_seg = seg;
-        }
-    }
-    *nseg = (faces + best_seg - 1) / best_seg;
-    return best_seg;
+    return segment_length(faces, blocks, slots, 2, 3, WK_SEG_MAX, nseg);
 }
 
 // cell index 0 (along DIR) of column `col` of the block's grid, clamped to
@@ -480,9 +470,10 @@ namespace cumc {
 // fluxes are bit-identical); lanes 2..28 then solve HLL at their faces. A
 // warp yields 27 faces; consecutive warps overlap by 5 cells. Loads and
 // stores are one 256-byte row segment per field.
-// Eight 128-thread blocks per SM (64 registers, a few spilled to L1): the
-// kernel is bound by FP64 dependency latency, and 32 resident warps hide more
-// of it than 20 unspilled ones (1.46 -> 1.25 ms at 256^3).
+// Eight 128-thread blocks per SM (64 registers, a few spilled to L1). The mixed
+// form's x sweep (bound by issue, 0.75 a cycle, and by its conversions: 0.70 ->
+// 0.66 ms a stage at 256^3 with branch-free roots) and the adjoint's face states;
+// in FP64 the two-cell form below is the default.
 // ---------------------------------------------------------------------------
 constexpr int XW_FACES = 27;
 
@@ -592,6 +583,11 @@ __device__ __forceinline__ void st_pair(R* p, int i, R a, R b, bool oka, bool ok
     }
 }
 
+__host__ __device__ __forceinline__ unsigned xpair_blocks(const Box& b) {
+    const unsigned warps = (unsigned)(b.SX * (b.ny + 2) - 2 + XP_FACES - 1) / XP_FACES;
+    return (warps + XP_THREADS / 32 - 1) / (XP_THREADS / 32);
+}
+
 // cell c's weights; TVD slopes count on 0..n+1 only, and beyond it the weights
 // of the nearest such cell keep them on the rounded path
 template <int RECON, typename R>
@@ -606,10 +602,12 @@ __global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ R sm[28][XP_THREADS];  // states of the pair's two faces: left 7, right 7 each
     const int cells = b.SX * (b.ny + 2);
-    const int w = blockIdx.x * (XP_THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31, tid = threadIdx.x;
+    const unsigned bpp = xpair_blocks(b), plane = blockIdx.x / bpp;  // blocks a plane
+    const int w = (int)(blockIdx.x - plane * bpp) * (XP_THREADS / 32) + (int)(threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, tid = threadIdx.x;
     if (w * XP_FACES + 2 >= cells || (b.skip && *b.skip)) return;  // uniform over the warp
     const int m = w * XP_FACES + 2 * lane;  // position of the lane's first cell in the plane's line
-    const int g = b.idx(-2, 0, l_lo + l_step * (int)blockIdx.y) + m;
+    const int g = b.idx(-2, 0, l_lo + l_step * (int)plane) + m;
     const int j0 = m % b.SX - 2, j1 = j0 == b.nx + 3 ? -2 : j0 + 1;
     const bool faces = lane >= 1 && lane <= 29;
     const bool ok0 = faces && m < cells && j0 >= 0 && j0 <= b.nx;
@@ -674,9 +672,6 @@ inline bool xpair_vec(const Box& b, const PrimT<R>& pr, const FaceFluxT<R>& out)
     for (int q = 0; q < 7; ++q) at |= (uintptr_t)out.f[q];
     return b.SX % 2 == 0 && at % (2 * sizeof(R)) == 0;
 }
-inline dim3 xpair_grid(const Box& b, int l_cnt) {
-    const int warps = (b.SX * (b.ny + 2) - 2 + XP_FACES - 1) / XP_FACES;
-    return dim3((unsigned)((warps + XP_THREADS / 32 - 1) / (XP_THREADS / 32)), (unsigned)l_cnt);
-}
+inline dim3 xpair_grid(const Box& b, int l_cnt) { return dim3(xpair_blocks(b) * (unsigned)l_cnt); }
 
 }  // namespace cumc

@@ -4,6 +4,7 @@ bit for bit against the FP64 oracle.
 
 * numerators that fade through the denormals (a faint velocity in a field at rest);
 * densities and pressures outside [2^-200, 2^200);
+* boxes longer than 65,535 planes or tiles of a grid dimension;
 * row lengths around multiples of the x sweep's 58 faces, odd and even, down
   to the smallest box.
 """
@@ -19,14 +20,14 @@ pytestmark = pytest.mark.gpu
 STEPS = 4
 
 
-def _check(p):
+def _check(p, steps=STEPS):
     from cumpic_b200.solver import CUMC3D
     from _oracle import Oracle
     g, o = CUMC3D(p), Oracle(p, threads=8)
     for s in (g, o):
         s.upload()
         s.initial_update()
-    for n in range(STEPS):
+    for n in range(steps):
         dg, do = g.finddt(), o.finddt()
         assert dg == do, (n, dg, do)
         g.rungekutta(dg)
@@ -57,3 +58,10 @@ def test_densities_outside_the_range(scale):
 @pytest.mark.parametrize("nx", [3, 4, 22, 23, 51, 52, 53, 58, 109, 110, 111, 168])
 def test_row_lengths(nx):
     _check(P.orszag_tang(nx, ny=5, nz=4))
+
+
+@pytest.mark.parametrize("axis,n", [(2, 65_600), (1, 262_200), (0, 70_000)], ids=["z", "y", "x"])
+def test_long_thin_boxes(axis, n):
+    shape = [3, 3, 3]
+    shape[axis] = n
+    _check(P.brio_wu(*shape, axis=axis), steps=1)
