@@ -186,7 +186,9 @@ struct CellWeights<1, double> {
     }
     __device__ __forceinline__ double slope(double vm, double vc, double vp) const {
         const double nf = 2.0 * (vp - vc), nb = 2.0 * (vc - vm);
-        if (!ok || tiny_min(nf, tiny_min(nb, ~0u)) < TINY) return tvd_slope(vm, vc, vp, cf, cb);
+        const unsigned mf = magnitude(nf), mb = magnitude(nb);
+        if (!ok || tiny_min(mf, tiny_min(mb, ~0u)) < TINY || max(mf, mb) >= HUGE_MAG)
+            return tvd_slope(vm, vc, vp, cf, cb);
         const double dqf = quot_signed(nf, cf, rf), dqb = quot_signed(nb, cb, rb);
         // (sign(dqf) + sign(dqb))/2 min(|dqf|, |dqb|), a zero positive where the signs differ
         const bool same = (__double2hiint(dqf) >= 0) == (__double2hiint(dqb) >= 0);

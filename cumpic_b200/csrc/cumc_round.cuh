@@ -36,11 +36,14 @@
 // two); their result depends on the seed, and the hardware's gives the rounded
 // root over both exponent parities (tests/test_round.py).
 //
-// Ranges: quotients need b in 2^+-500 and |a| zero or at least 2^-900 (the
-// remainder must not be rounded); roots need a in 2^+-900.
+// Ranges: a quotient needs b in 2^+-500, a finite, and a/b, unless a is zero, a
+// normal number with its remainder above the subnormal ones; roots need a in
+// 2^+-900. quot_group tests b in [2^-200, 2^200) and |a| zero or in
+// [2^-800, 2^800), so that a/b lies in 2^+-1000.
 #pragma once
 #include <cfenv>
 #include <cmath>
+#include <cstring>
 #ifdef __CUDACC__
 #define CUMC_HD __host__ __device__ __forceinline__
 #else
@@ -94,61 +97,115 @@ CUMC_HD double root_refine(double a, double y0) {
     return std::fma(std::fma(-g, g, a), h, g);
 }
 
-#ifdef __CUDACC__
-__device__ __forceinline__ double recip_seed(double b) {
+// the approximate reciprocal (on the host, where only the tests come, with a
+// relative error of the same size)
+CUMC_HD double recip_seed(double b) {
+#ifdef __CUDA_ARCH__
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     return y;
+#else
+    return 1.0 / b * (1.0 + 0x1p-20);
+#endif
 }
-__device__ __forceinline__ double rsqrt_seed(double a) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    return y;
-}
-__device__ __forceinline__ Recip recip_of(double b) { return recip_refine(b, recip_seed(b)); }
-__device__ __forceinline__ double root_of(double a) { return root_refine(a, rsqrt_seed(a)); }
-// sqrt(max(a, 0))
-__device__ __forceinline__ double root_pos(double a) { return __double_as_longlong(a) > 0 ? root_of(a) : 0.0; }
+CUMC_HD Recip recip_of(double b) { return recip_refine(b, recip_seed(b)); }
 // a/b with a zero's sign kept; b > 0
-__device__ __forceinline__ double quot_signed(double a, double b, const Recip& r) {
-    return copysign(quot(a, b, r), a);
-}
+CUMC_HD double quot_signed(double a, double b, const Recip& r) { return std::copysign(quot(a, b, r), a); }
 
-// out-of-range tracking on the high words, integer pipe only:
+// Out-of-range tracking on the two words of a double, integer pipe only (one
+// instruction each for the sums with a minimum or maximum)
+CUMC_HD unsigned hi_word(double x) {
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2hiint(x);
+#else
+    unsigned long long u;
+    std::memcpy(&u, &x, sizeof u);
+    return (unsigned)(u >> 32);
+#endif
+}
+CUMC_HD unsigned lo_word(double x) {
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2loint(x);
+#else
+    unsigned long long u;
+    std::memcpy(&u, &x, sizeof u);
+    return (unsigned)u;
+#endif
+}
+CUMC_HD unsigned add_max(unsigned a, unsigned b, unsigned m) {
+#ifdef __CUDA_ARCH__
+    return __viaddmax_u32(a, b, m);
+#else
+    return a + b > m ? a + b : m;
+#endif
+}
+CUMC_HD unsigned add_min(unsigned a, unsigned b, unsigned m) {
+#ifdef __CUDA_ARCH__
+    return __viaddmin_u32(a, b, m);
+#else
+    return a + b < m ? a + b : m;
+#endif
+}
 // range_max accumulates max(hi - lo_word) so that one unsigned compare covers
-// several positive operands; tiny_min accumulates the smallest nonzero
-// magnitude (a zero counts as the largest)
+// several positive operands. magnitude orders a double by its size (twice the
+// high word, and one for low bits: 0 for a zero alone, an infinity or a NaN above
+// every number); tiny_min accumulates the smallest nonzero one less one (a zero
+// counts as the largest)
 constexpr unsigned RANGE_LO = (1023u - 200u) << 20, RANGE_SPAN = 400u << 20;  // [2^-200, 2^200)
-__device__ __forceinline__ unsigned range_max(double x, unsigned m) {
-    return __viaddmax_u32((unsigned)__double2hiint(x), 0u - RANGE_LO, m);
+CUMC_HD unsigned range_max(double x, unsigned m) { return add_max(hi_word(x), 0u - RANGE_LO, m); }
+constexpr unsigned TINY = ((1023u - 800u) << 21) - 1u;  // 2^-800's magnitude, less one
+constexpr unsigned HUGE_MAG = (1023u + 800u) << 21;     // 2^800's
+CUMC_HD unsigned magnitude(double x) {
+    const unsigned hi = hi_word(x), lo = lo_word(x);
+    return hi + hi + (lo < 1u ? lo : 1u);
 }
-constexpr unsigned TINY = ((1023u - 900u) << 21) - 1u;  // twice the high word of 2^-900, less one
-__device__ __forceinline__ unsigned tiny_min(double x, unsigned m) {
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    return __viaddmin_u32(hi + hi + min(lo, 1u), ~0u, m);
-}
+CUMC_HD unsigned tiny_min(unsigned mag, unsigned m) { return add_min(mag, ~0u, m); }
 
 // a/b out of line, for the rare groups below
-static __device__ __noinline__ double plain_quot(double a, double b) { return a / b; }
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__ double plain_quot(double a, double b) { return a / b; }
+#else
+inline double plain_quot(double a, double b) { return a / b; }
+#endif
 
 // q[n] = a[n]/b for N numerators, the shared reciprocal
 // where b and the numerators are in range, else the plain operator
 // (a front that fades into a zero field carries numerators down through the
 // denormals, so the test stands here and not around a whole face or cell)
 template <int N>
-__device__ __forceinline__ void quot_group(const double (&a)[N], double b, double (&q)[N]) {
-    unsigned tiny = ~0u;
+CUMC_HD void quot_group(const double (&a)[N], double b, double (&q)[N]) {
+    unsigned tiny = ~0u, huge = 0u;
+#ifdef __CUDA_ARCH__
 #pragma unroll
-    for (int n = 0; n < N; ++n) tiny = tiny_min(a[n], tiny);
-    if (range_max(b, 0u) < RANGE_SPAN && tiny >= TINY) {
+#endif
+    for (int n = 0; n < N; ++n) {
+        const unsigned mag = magnitude(a[n]);
+        tiny = tiny_min(mag, tiny);
+        huge = mag > huge ? mag : huge;
+    }
+    if (range_max(b, 0u) < RANGE_SPAN && tiny >= TINY && huge < HUGE_MAG) {
         const Recip r = recip_of(b);
+#ifdef __CUDA_ARCH__
 #pragma unroll
+#endif
         for (int n = 0; n < N; ++n) q[n] = quot_signed(a[n], b, r);
     } else {
+#ifdef __CUDA_ARCH__
 #pragma unroll
+#endif
         for (int n = 0; n < N; ++n) q[n] = plain_quot(a[n], b);
     }
 }
+
+#ifdef __CUDACC__
+__device__ __forceinline__ double rsqrt_seed(double a) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    return y;
+}
+__device__ __forceinline__ double root_of(double a) { return root_refine(a, rsqrt_seed(a)); }
+// sqrt(max(a, 0))
+__device__ __forceinline__ double root_pos(double a) { return __double_as_longlong(a) > 0 ? root_of(a) : 0.0; }
 
 // FP32 reciprocal and root, rounded to nearest (the results of 1.0f/x and
 // sqrtf, checked over every significand by the tests): one Newton step from
