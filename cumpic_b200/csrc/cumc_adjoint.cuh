@@ -626,7 +626,7 @@ __device__ __forceinline__ PpmSlope ppm_slope_grad(double vm, double vc, double 
     const double delta = b0 * up + b1 * dn;
     const double m1 = fabs(delta), hd = fabs(dn), hu = fabs(up);
     const double m2 = 2.0 * hd, m3 = 2.0 * hu, m12 = min_mag(m1, m2);
-    const bool on = is_pos(up * dn);
+    const bool on = above_zero<true>(up * dn);
     const bool by_up = m12 > m3, by_dn = !by_up && m1 > m2;  // limited by 2 |vc - vp|, by 2 |vc - vm|
     // sd 2 sign(dn); sign(up) = sign(dn) where the slope is on
     const double g = copysign(2.0, delta) * copysign(1.0, dn);
@@ -642,10 +642,10 @@ struct PpmFixAdj {
 };
 __device__ __forceinline__ PpmFixAdj ppm_fix_adj(double vc, double vl, double vr, double lvm, double lvp) {
     const double c3 = 3.0 * vc;
-    const bool flat = !is_pos((vr - vc) * (vc - vl));
-    const bool t1 = is_neg((vr - vl) * __fma_rn(2.0, vr, vl - c3));
+    const bool flat = not_above_zero<true>((vr - vc) * (vc - vl));
+    const bool t1 = below_zero<true>((vr - vl) * __fma_rn(2.0, vr, vl - c3));
     const double vm = t1 ? __fma_rn(-2.0, vr, c3) : vl;
-    const bool t2 = is_neg((vr - vm) * (__fma_rn(-2.0, vl, c3) - vr));
+    const bool t2 = below_zero<true>((vr - vm) * (__fma_rn(-2.0, vl, c3) - vr));
     const double m1 = t1 ? lvm : 0.0, p1 = t2 ? lvp : 0.0;  // seeds that the fixes took over
     PpmFixAdj a;
     a.c = flat ? lvm + lvp : 3.0 * (m1 + p1);

@@ -197,13 +197,13 @@ template <int RECON, typename R>
 __device__ __forceinline__ void walk_prologue(const AxisTabs& A, int f0, R x0, R x1, R x2, R x3, R x4, R& vpf, R& d1,
                                               R& Vf) {
     if (RECON == 4) {
-        const R dm0 = ppm_slope(x0, x1, x2, (R)A.s0[f0 - 1], (R)A.s1[f0 - 1]);
-        const R dmc = ppm_slope(x1, x2, x3, (R)A.s0[f0], (R)A.s1[f0]);
-        const R dmp = ppm_slope(x2, x3, x4, (R)A.s0[f0 + 1], (R)A.s1[f0 + 1]);
+        const R dm0 = ppm_slope<false>(x0, x1, x2, (R)A.s0[f0 - 1], (R)A.s1[f0 - 1]);
+        const R dmc = ppm_slope<false>(x1, x2, x3, (R)A.s0[f0], (R)A.s1[f0]);
+        const R dmp = ppm_slope<false>(x2, x3, x4, (R)A.s0[f0 + 1], (R)A.s1[f0 + 1]);
         const R Vm = ppm_face(x1, x2, dm0, dmc, (R)A.a0[f0 - 1], (R)A.a1[f0 - 1], (R)A.a2[f0 - 1], (R)A.a3[f0 - 1]);
         const R Vp = ppm_face(x2, x3, dmc, dmp, (R)A.a0[f0], (R)A.a1[f0], (R)A.a2[f0], (R)A.a3[f0]);
         R vm, vp;
-        ppm_fix(x2, Vm, Vp, vm, vp);
+        ppm_fix<false>(x2, Vm, Vp, vm, vp);
         vpf = vp;
         d1 = dmp;
         Vf = Vp;
@@ -229,9 +229,9 @@ template <int RECON, typename R>
 __device__ __forceinline__ void walk_step(const CellWeights<RECON, R>& W, R v0, R v1, R v2, R x, R& d1, R& Vf, R& vm1,
                                           R& vp1) {
     if constexpr (RECON == 4) {
-        const R d2 = W.slope(v1, v2, x);
+        const R d2 = W.template slope<false>(v1, v2, x);
         const R Vn = W.face(v1, v2, d1, d2);
-        ppm_fix(v1, Vf, Vn, vm1, vp1);
+        ppm_fix<false>(v1, Vf, Vn, vm1, vp1);
         d1 = d2;
         Vf = Vn;
     } else {

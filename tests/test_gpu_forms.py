@@ -1,0 +1,207 @@
+"""The branch-free forms of the limiter, the HLL solve and the CFL step against
+the plain operators they stand for, over states that leave the forms' ranges:
+overflowing, infinite and not-a-number values, faint fields, zero pressure. A
+test kernel evaluates both on the same operands."""
+import ctypes
+import itertools
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cumpic_b200", "csrc")
+GGAS = 5.0 / 3.0
+
+SRC = """
+#include "%s/cumc_kernels.cuh"
+using namespace cumc;
+template <int DIR, typename R, bool RECIP>
+__global__ void k_hll(long n, const R* w, R g, R* out, R* ref, R* scale) {
+    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    R wl[8], wr[8], f[7], p[7];
+    for (int q = 0; q < 8; ++q) wl[q] = w[16 * i + q], wr[q] = w[16 * i + 8 + q];
+    sweep_hll<DIR, R, RECIP>(wl, wr, g, f);
+    if constexpr (sizeof(R) == 4) hll_flux7_mixed_form<DIR, false>(wl, wr, g, p);
+    else hll_flux7<DIR, R>(wl, wr, g, p);
+    for (int q = 0; q < 7; ++q) out[7 * i + q] = f[q], ref[7 * i + q] = p[q];
+    // the largest flux and signal speed times conserved value that enter
+    const FaceSide<DIR, R> L(wl, g), S(wr, g);
+    for (int q = 0, c = 0; q < 8; ++q) {
+        if (q == IBX + DIR) continue;
+        const R cl = sqrt(g * wl[4] / wl[0] + (2 * L.hb2) / wl[0]) + fabs(wl[IVX + DIR]);
+        const R cr = sqrt(g * wr[4] / wr[0] + (2 * S.hb2) / wr[0]) + fabs(wr[IVX + DIR]);
+        scale[7 * i + c++] = fabs(L.f(q)) + fabs(S.f(q)) + fmax(cl, cr) * (fabs(L.u(q)) + fabs(S.u(q)));
+    }
+}
+template <typename R, bool RECIP>
+int run_hll(int dir, long n, const R* w, R g, R* out) {
+    R *dw, *d;
+    if (cudaMalloc(&dw, 16 * n * sizeof(R)) || cudaMalloc(&d, 21 * n * sizeof(R))) return 1;
+    cudaMemcpy(dw, w, 16 * n * sizeof(R), cudaMemcpyHostToDevice);
+    const unsigned b = (unsigned)((n + 127) / 128);
+    if (dir == 0) k_hll<0, R, RECIP><<<b, 128>>>(n, dw, g, d, d + 7 * n, d + 14 * n);
+    if (dir == 1) k_hll<1, R, RECIP><<<b, 128>>>(n, dw, g, d, d + 7 * n, d + 14 * n);
+    if (dir == 2) k_hll<2, R, RECIP><<<b, 128>>>(n, dw, g, d, d + 7 * n, d + 14 * n);
+    const int rc = cudaMemcpy(out, d, 21 * n * sizeof(R), cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(dw), cudaFree(d);
+    return rc;
+}
+extern "C" int hll_rounded(int dir, long n, const double* w, double g, double* out) { return run_hll<double, false>(dir, n, w, g, out); }
+extern "C" int hll_recip(int dir, long n, const double* w, double g, double* out) { return run_hll<double, true>(dir, n, w, g, out); }
+extern "C" int hll_mixed(int dir, long n, const float* w, float g, float* out) { return run_hll<float, false>(dir, n, w, g, out); }
+
+__global__ void k_dt(long n, const double* w, double g, double cfl, const double* d, double* out) {
+    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    Tabs T{};
+    for (int a = 0; a < 3; ++a) T.ax[a].d = d + a;
+    const double* c = w + 8 * i;
+    out[i] = cell_dt_rounded<1>(T, 0, 0, 0, c[0], c[4], c[1], c[2], c[3], c[5], c[6], c[7], g, cfl);
+    out[n + i] = cfl_cell_dt(c[0], c[4], c[1], c[2], c[3], c[5], c[6], c[7], d[0], d[1], d[2], g, cfl);
+}
+extern "C" int cfl(long n, const double* w, double g, double number, const double* widths, double* out) {
+    double *dw, *d;
+    if (cudaMalloc(&dw, (8 * n + 3) * sizeof(double)) || cudaMalloc(&d, 2 * n * sizeof(double))) return 1;
+    cudaMemcpy(dw, w, 8 * n * sizeof(double), cudaMemcpyHostToDevice);
+    cudaMemcpy(dw + 8 * n, widths, 3 * sizeof(double), cudaMemcpyHostToDevice);
+    k_dt<<<(unsigned)((n + 127) / 128), 128>>>(n, dw, g, number, dw + 8 * n, d);
+    const int rc = cudaMemcpy(out, d, 2 * n * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(dw), cudaFree(d);
+    return rc;
+}
+
+// x: five cells, then two weights of a slope and (cf, cb) of a TVD cell
+__global__ void k_limit(long n, const double* x, double* out) {
+    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double* v = x + 9 * i;
+    out[i] = ppm_slope(v[1], v[2], v[3], v[5], v[6]);
+    ppm_fix(v[2], v[1], v[3], out[n + i], out[2 * n + i]);
+    AxisTabs A{};
+    A.tcf = v + 7;
+    A.tcb = v + 8;
+    out[3 * n + i] = CellWeights<1, double>(A, 0).slope(v[1], v[2], v[3]);
+}
+extern "C" int limit(long n, const double* x, double* out) {
+    double *dx, *d;
+    if (cudaMalloc(&dx, 9 * n * sizeof(double)) || cudaMalloc(&d, 4 * n * sizeof(double))) return 1;
+    cudaMemcpy(dx, x, 9 * n * sizeof(double), cudaMemcpyHostToDevice);
+    k_limit<<<(unsigned)((n + 127) / 128), 128>>>(n, dx, d);
+    const int rc = cudaMemcpy(out, d, 4 * n * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(dx), cudaFree(d);
+    return rc;
+}
+""" % CSRC
+
+
+def _build(d, name, flags):
+    src, so = d / (name + ".cu"), d / (name + ".so")
+    src.write_text(SRC)
+    subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", *flags, "-shared",
+                    "-Xcompiler", "-fPIC", "-o", str(so), str(src)], check=True)
+    return ctypes.CDLL(str(so))
+
+
+@pytest.fixture(scope="module")
+def lib64(tmp_path_factory):
+    from cumpic_b200.build import FP64_FLAGS
+    return _build(tmp_path_factory.mktemp("forms"), "f64", FP64_FLAGS)
+
+
+@pytest.fixture(scope="module")
+def lib32(tmp_path_factory):
+    from cumpic_b200.build import MIXED_FLAGS
+    return _build(tmp_path_factory.mktemp("forms"), "f32", MIXED_FLAGS)
+
+
+def _p(a):
+    return a.ctypes.data_as(ctypes.c_void_p)
+
+
+def _same(x, y):
+    """the same bits, any NaN equal to any other"""
+    kind = np.int64 if x.dtype == np.float64 else np.int32
+    return (x.view(kind) == y.view(kind)) | (np.isnan(x) & np.isnan(y))
+
+
+def ordinary(n, rng, dtype):
+    """states (rho, v, p, B) of order one"""
+    w = rng.uniform(-1.0, 1.0, (n, 8))
+    w[:, 0] = rng.uniform(0.1, 1.0, n)
+    w[:, 4] = rng.uniform(0.1, 1.0, n)
+    return w.astype(dtype)
+
+
+def edge_states(dtype, specials, scales, seed):
+    """pairs of states: one value of either side replaced by each special one;
+    densities, pressures and fields of either side scaled"""
+    rng = np.random.default_rng(seed)
+    out = []
+    for side, q, s in itertools.product((0, 1), range(8), specials):
+        w = ordinary(40, rng, dtype).reshape(20, 2, 8)
+        w[:, side, q] = dtype(s)
+        w[10:, side, q] *= dtype(-1)
+        out.append(w)
+    for a, b, c in itertools.product(scales, scales, scales):
+        w = ordinary(16, rng, np.float64).reshape(8, 2, 8)
+        w[:, :, 0] *= a
+        w[:, :, 4] *= b
+        w[:, :, 5:] *= c
+        out.append(w.astype(dtype))
+    return np.ascontiguousarray(np.concatenate(out).reshape(-1, 16))
+
+
+with np.errstate(over="ignore"):
+    SPECIAL64 = [0.0, np.inf, np.nan, 5e-324, 1e-310, 1e-300, 1e-162, 1e-154, 1e-80, 1e-70, 1e-30, 1e30, 1e75, 1e80,
+                 1e130, 1e153, 1e155, 1e200, 1.7e308]
+    SCALE64 = [0.0, 1e-300, 1e-160, 1e-78, 1e-61, 1.0, 1e61, 1e78, 1e140, 1e160]
+    SPECIAL32 = [0.0, np.inf, np.nan, 1e-45, 1e-38, 1e-30, 1e-19, 1e-12, 1e-9, 1e9, 1e10, 1e15, 1e19, 1e20, 3e38]
+    SCALE32 = [0.0, 1e-38, 1e-20, 1e-18, 1e-12, 1.0, 1e10, 1e13, 1e19, 1e30]
+
+
+def _hll(run, w, g, dtype):
+    n = len(w)
+    out = np.empty((3, n, 7), dtype)
+    res = []
+    for d in range(3):
+        assert run(d, ctypes.c_long(n), _p(w), g, _p(out)) == 0
+        res.append(out.copy())
+    return res
+
+
+def test_limiter_is_the_plain_one(lib64):
+    """values up to 1e300 (their triples stay finite) or infinite or NaN"""
+    rng = np.random.default_rng(3)
+    special = [0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, -1e-310, 1e-300, 1e300, -1e300]
+    x = rng.uniform(-1.0, 1.0, (4000 + 40 * 3 * len(special), 9))
+    x[:2000, :5] *= 10.0 ** rng.integers(-300, 300, 2000)[:, None]
+    at = 4000
+    for q, s in itertools.product((1, 2, 3), special):
+        x[at:at + 40, q] = s
+        x[at + 20:at + 30, 1 + q % 3] = s  # and a second cell
+        at += 40
+    x[:, 5:7] = rng.uniform(0.2, 0.8, (len(x), 2))
+    x[:, 7:] = rng.uniform(0.1, 3.0, (len(x), 2))
+    x = np.ascontiguousarray(x)
+    out = np.empty((4, len(x)))
+    assert lib64.limit(ctypes.c_long(len(x)), _p(x), _p(out)) == 0
+    vm, vc, vp, b0, b1, cf, cb = x[:, [1, 2, 3, 5, 6, 7, 8]].T
+    with np.errstate(all="ignore"):
+        up, dn = vp - vc, vc - vm
+        delta = b0 * up + b1 * dn
+        slope = np.where(up * dn > 0.0, np.fmin(np.fmin(np.abs(delta), 2 * np.abs(dn)), 2 * np.abs(vc - vp))
+                         * np.copysign(1.0, delta), 0.0)
+        vl, vr = vm, vp
+        flat = (vr - vc) * (vc - vl) <= 0.0
+        m = np.where((vr - vl) * ((vl - 3.0 * vc) + 2.0 * vr) < 0.0, 3.0 * vc - 2.0 * vr, vl)
+        p = np.where((vr - m) * ((3.0 * vc - 2.0 * vl) - vr) < 0.0, 3.0 * vc - 2.0 * vl, vr)
+        f, b = 2.0 * up / cf, 2.0 * dn / cb
+        tvd = (0.5 * (np.copysign(1.0, f) + np.copysign(1.0, b))) * np.fmin(np.abs(f), np.abs(b))
+    for name, got, want in (("slope", out[0], slope), ("lower", out[1], np.where(flat, vc, m)),
+                            ("upper", out[2], np.where(flat, vc, p)), ("tvd", out[3], tvd)):
+        bad = ~_same(got, want)
+        assert not bad.any(), (name, bad.sum(), x[bad][0], got[bad][0], want[bad][0])
