@@ -402,10 +402,26 @@ __device__ __noinline__ void hll_flux7_ieee(const double* w, double ggas, double
     for (int q = 0; q < 7; ++q) out[q] = fx[q];
 }
 
+// Bounds of the branch-free solves. With densities and pressures in
+// [2^-200, 2^200), a squared sound speed is at least 2^-400; with a2 + b2 below
+// 2^500 every square, root and quotient of the speeds is a normal number (a
+// faint field's share of a sum below 2^-900 vanishes beside a2, whatever its
+// quotient), and with normal velocities below 2^500 so are the Roe averages. An
+// overflow, an infinity or a NaN on the way leaves a2 + b2 or the velocity
+// above its bound, since every word of it compares as more than any number's.
+constexpr unsigned SQUARE_MAX = (1023u + 500u) << 20;   // the high word of 2^500
+constexpr unsigned SPEED_MAX = SQUARE_MAX << 1;         // without the sign
+__device__ __forceinline__ unsigned speed_max(double vl, double vr) {
+    const unsigned l = hi_word(vl), r = hi_word(vr);
+    return max(l + l, r + r);
+}
+
 // one side's fast speed and internal energy for hll_flux7_rounded; the values
-// of EOS_SOUNDSPEED, compute_signalspeed and EOS_EPSILON
+// of EOS_SOUNDSPEED, compute_signalspeed and EOS_EPSILON; square: high word of
+// a2 + b2
 struct SideSpeed {
     double cf, sq, e;
+    unsigned square;
 };
 __device__ __forceinline__ SideSpeed side_speed(double rho, double p, double bn2, double bt1, double bt2, double ggas,
                                                 double gm1, const Recip& rg) {
@@ -417,7 +433,7 @@ __device__ __forceinline__ SideSpeed side_speed(double rho, double p, double bn2
     // ((a4 + b4) + (2 b2) a2) - (4 a2) b2n with the exact factors 2 and 4 merged
     const double x = __fma_rn(2.0, b2 * a2, a2 * a2 + b2 * b2);
     const double s = root_pos(__fma_rn(-4.0, a2 * b2n, x));
-    return {root_of(0.5 * ((a2 + b2) + s)), root_of(rho), quot(quot(p, rho, r), gm1, rg)};
+    return {root_of(0.5 * ((a2 + b2) + s)), root_of(rho), quot(quot(p, rho, r), gm1, rg), hi_word(a2 + b2)};
 }
 
 // hll_flux7 in FP64, bit for bit, with the quotients and roots of
@@ -426,24 +442,24 @@ __device__ __forceinline__ SideSpeed side_speed(double rho, double p, double bn2
 // kept them from overlapping (1,414 instructions a face and warp in the y
 // walker, 0.53 issued a cycle at 160^3). y and z walkers 1.17 -> 0.88 ms and the
 // x sweep 1.25 -> 1.08 ms at 256^3 with the integer-pipe limiter above; the
-// torus' y walker 0.193 -> 0.108 ms. Returns false where a density or pressure
-// lies outside [2^-200, 2^200) and the face needs the plain operators
-// throughout. (Squared fields below 2^-900 need no test: they vanish in the
-// sums with a2 >= 2^-402.)
+// torus' y walker 0.193 -> 0.108 ms. Returns false where a density, a pressure,
+// gamma - 1, a squared speed or a normal velocity lies outside the bounds above
+// and the face needs the plain operators throughout.
 template <int DIR>
 __device__ __forceinline__ bool hll_flux7_rounded(const double (&wl)[8], const double (&wr)[8], double ggas,
                                                   double (&out)[7]) {
     constexpr int ivn = IVX + DIR, ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
     constexpr int bt_a = DIR == 0 ? IBY : IBX, bt_b = DIR == 2 ? IBY : IBZ;
     constexpr int comp[7] = {IRHO, IVX, IVY, IVZ, ITAU, bt_a, bt_b};
-    const unsigned far =
-        range_max(wl[IRHO], range_max(wr[IRHO], range_max(wl[ITAU], range_max(wr[ITAU], 0u))));
-    if (far >= RANGE_SPAN) return false;
-    using Side = FaceSide<DIR, double>;
     const double gm1 = ggas - 1.0, bn2 = wl[ibn] * wl[ibn];
+    const unsigned far =
+        range_max(wl[IRHO], range_max(wr[IRHO], range_max(wl[ITAU], range_max(wr[ITAU], range_max(gm1, 0u)))));
+    if (far >= RANGE_SPAN || speed_max(wl[ivn], wr[ivn]) >= SPEED_MAX) return false;
+    using Side = FaceSide<DIR, double>;
     const Recip rg = recip_of(gm1);
     const SideSpeed l = side_speed(wl[IRHO], wl[ITAU], bn2, wl[ibt1], wl[ibt2], ggas, gm1, rg);
     const SideSpeed r = side_speed(wr[IRHO], wr[ITAU], bn2, wr[ibt1], wr[ibt2], ggas, gm1, rg);
+    if (max(l.square, r.square) >= SQUARE_MAX) return false;
     const double sq = l.sq + r.sq;
     const Recip rs = recip_of(sq);
     const double ubar = quot(l.sq * wl[ivn] + r.sq * wr[ivn], sq, rs);

@@ -626,20 +626,20 @@ __device__ __forceinline__ void st2(double* p, int i, double x, double y) {
 }
 
 // cell_dt with the quotients and roots of cumc_round.cuh: the same value
-// bit for bit, by the plain operators outside their ranges
+// bit for bit, by the plain operators outside the bounds of hll_flux7_rounded
 template <int COORD>
 __device__ __forceinline__ double cell_dt_rounded(const Tabs& T, int j, int k, int l, double rho, double p, double vx,
                                                   double vy, double vz, double bcx, double bcy, double bcz,
                                                   double ggas, double cfl) {
-    if (range_max(rho, range_max(p, 0u)) >= RANGE_SPAN)
-        return cell_dt<COORD>(T, j, k, l, rho, p, vx, vy, vz, bcx, bcy, bcz, ggas, cfl);
-    double dyl = T.ax[1].d[k], dzl = T.ax[2].d[l];
-    if (COORD != 1) cfl_lengths(COORD, T.ax[0].c[j], COORD == 3 ? T.sinc[k] : 0.0, dyl, dzl);
     const Recip r = recip_of(rho);
     const double cs = root_of(quot(ggas * p, rho, r));
     const double a2 = cs * cs;
     const double b2x = quot(bcx * bcx, rho, r), b2y = quot(bcy * bcy, rho, r), b2z = quot(bcz * bcz, rho, r);
     const double b2 = (b2x + b2y) + b2z;
+    if (range_max(rho, range_max(p, 0u)) >= RANGE_SPAN || hi_word(a2 + b2) >= SQUARE_MAX)
+        return cell_dt<COORD>(T, j, k, l, rho, p, vx, vy, vz, bcx, bcy, bcz, ggas, cfl);
+    double dyl = T.ax[1].d[k], dzl = T.ax[2].d[l];
+    if (COORD != 1) cfl_lengths(COORD, T.ax[0].c[j], COORD == 3 ? T.sinc[k] : 0.0, dyl, dzl);
     const double base = __fma_rn(2.0, a2 * b2, a2 * a2) + b2 * b2;
     auto fast = [&](double b2d) {  // no MAX(., 0) under the inner root, as in cfl_cell_dt
         const double x = __fma_rn(-4.0, a2 * b2d, base);

@@ -24,6 +24,7 @@ __global__ void k_hll(long n, const R* w, R g, R* out, R* ref, R* scale) {
     if (i >= n) return;
     R wl[8], wr[8], f[7], p[7];
     for (int q = 0; q < 8; ++q) wl[q] = w[16 * i + q], wr[q] = w[16 * i + 8 + q];
+    wr[IBX + DIR] = wl[IBX + DIR];  // one normal field a face
     sweep_hll<DIR, R, RECIP>(wl, wr, g, f);
     if constexpr (sizeof(R) == 4) hll_flux7_mixed_form<DIR, false>(wl, wr, g, p);
     else hll_flux7<DIR, R>(wl, wr, g, p);
@@ -171,6 +172,23 @@ def _hll(run, w, g, dtype):
         assert run(d, ctypes.c_long(n), _p(w), g, _p(out)) == 0
         res.append(out.copy())
     return res
+
+
+def test_hll_rounded_is_the_plain_solve(lib64):
+    w = edge_states(np.float64, SPECIAL64, SCALE64, 1)
+    for d, (f, ref, _) in enumerate(_hll(lib64.hll_rounded, w, ctypes.c_double(GGAS), np.float64)):
+        bad = ~_same(f, ref).all(axis=1)
+        assert not bad.any(), (d, bad.sum(), w[bad][0], f[bad][0], ref[bad][0])
+
+
+def test_cfl_rounded_is_the_plain_step(lib64):
+    w = edge_states(np.float64, SPECIAL64, SCALE64, 2).reshape(-1, 8)
+    out = np.empty((2, len(w)))
+    widths = np.array([0.1, 0.2, 0.3])
+    assert lib64.cfl(ctypes.c_long(len(w)), _p(w), ctypes.c_double(GGAS), ctypes.c_double(0.4), _p(widths),
+                     _p(out)) == 0
+    bad = ~_same(out[0], out[1])
+    assert not bad.any(), (bad.sum(), w[bad][0], out[:, bad][:, 0])
 
 
 def test_limiter_is_the_plain_one(lib64):
