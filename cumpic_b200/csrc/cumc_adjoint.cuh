@@ -190,9 +190,9 @@ __device__ __forceinline__ SideWave<DIR> side_wave(const double (&w)[8], double 
         root = root_pos(inner);
         s.cf = root_of(0.5 * ((s.a2 + s.b2) + root));
         s.sq = root_of(rho);
-        s.is = inner > 0.0 ? recip_r(root) : 0.0;
-        s.icf = recip_r(s.cf);
-        s.ics_p = recip_r(p);
+        s.is = inner > 0.0 ? recip_q<true>(root) : 0.0;
+        s.icf = recip_q<true>(s.cf);
+        s.ics_p = recip_q<true>(p);
     } else {
         s.irho = 1.0 / rho;
         s.cs = sqrt((g * p) / rho);
@@ -230,7 +230,7 @@ __device__ __forceinline__ void hll_adj(const double (&wl)[8], const double (&wr
     constexpr int bt_a = DIR == 0 ? IBY : IBX;
     constexpr int bt_b = DIR == 2 ? IBY : IBZ;
     constexpr int comp[7] = {IRHO, IVX, IVY, IVZ, ITAU, bt_a, bt_b};
-    const double ig1 = recip_r(g - 1.0);
+    const double ig1 = recip_q<true>(g - 1.0);
     SideWave<DIR> w[2];
     if (range_max(wl[IRHO], range_max(wr[IRHO], range_max(wl[ITAU], range_max(wr[ITAU], 0u)))) < RANGE_SPAN) {
         w[0] = side_wave<DIR, true>(wl, g);
@@ -253,7 +253,7 @@ __device__ __forceinline__ void hll_adj(const double (&wl)[8], const double (&wr
     const double sL = fmin(aL, bL), sR = fmax(aR, bR);
     double ln[7], kf[2], ku[2], lsL = 0.0, lsR = 0.0;
     const bool mid = !(sL >= 0.0) && sR >= 0.0;
-    const double id = mid ? recip_r(sR - sL) : 1.0;
+    const double id = mid ? recip_q<true>(sR - sL) : 1.0;
 #pragma unroll
     for (int c = 0; c < 7; ++c) ln[c] = lout[c] * id;
     kf[0] = mid ? sR : sL >= 0.0 ? 1.0 : 0.0;

@@ -231,31 +231,40 @@ __device__ __forceinline__ R signalspeed(R cs, R bn, R bt1, R bt2, R rho) {
     return sqrt(R(0.5) * ((a2 + b2) + sqrt(fmax(((a4 + b4) + (R(2) * b2) * a2) - (R(4) * a2) * b2n, R(0)))));
 }
 
-// 1/x, sqrt(x) and sqrt(max(x, 0)) of the reciprocal form: in FP64 by
-// Newton-Raphson without a branch (within a unit in the last place), in FP32
-// the IEEE operations
-__device__ __forceinline__ double recip_r(double x) { return recip_near(x, recip_seed(x)); }
-__device__ __forceinline__ float recip_r(float x) { return 1.0f / x; }
-// FP32 with (ROUNDED) and without the branch-free forms: the same values where
-// hll_flux7_mixed's range test holds
-template <bool ROUNDED>
-__device__ __forceinline__ float recip_q(float x) { return ROUNDED ? recip_f(x) : 1.0f / x; }
-template <bool ROUNDED>
-__device__ __forceinline__ float root_q(float x) { return ROUNDED ? root_f(x) : sqrtf(x); }
-template <bool ROUNDED>
+// 1/x, sqrt(x) and sqrt(max(x, 0)) of the reciprocal forms. NEAR: without a
+// branch, for the operands that the callers' range tests admit: in FP32 the
+// IEEE results, in FP64 the reciprocal within a unit in the last place and the
+// IEEE root. Else the IEEE operations.
+template <bool NEAR>
+__device__ __forceinline__ float recip_q(float x) { return NEAR ? recip_f(x) : 1.0f / x; }
+template <bool NEAR>
+__device__ __forceinline__ double recip_q(double x) {
+    if constexpr (NEAR) return recip_near(x, recip_seed(x));
+    return 1.0 / x;
+}
+template <bool NEAR>
+__device__ __forceinline__ float root_q(float x) { return NEAR ? root_f(x) : sqrtf(x); }
+template <bool NEAR>
+__device__ __forceinline__ double root_q(double x) {
+    if constexpr (NEAR) return root_of(x);
+    return sqrt(x);
+}
+template <bool NEAR>
 __device__ __forceinline__ float root_max0_q(float x) {
-    if (!ROUNDED) return sqrtf(fmaxf(x, 0.0f));
+    if (!NEAR) return sqrtf(fmaxf(x, 0.0f));
     return x > 0.0f ? root_f(x) : 0.0f;
 }
-__device__ __forceinline__ double sqrt_r(double x) { return root_pos(x); }
-__device__ __forceinline__ float sqrt_r(float x) { return sqrtf(x); }
-__device__ __forceinline__ double sqrt_max0(double x) { return root_pos(x); }
-__device__ __forceinline__ float sqrt_max0(float x) { return sqrtf(fmaxf(x, 0.0f)); }
+template <bool NEAR>
+__device__ __forceinline__ double root_max0_q(double x) {
+    if constexpr (NEAR) return root_pos(x);
+    return sqrt(fmax(x, 0.0));
+}
 
 // compute_signalspeed with the quotients by rho formed as products with
-// irho = 1/rho (the CUMC_FP64_FAST form: not bit-compatible with the reference)
-template <typename R>
-__device__ __forceinline__ R signalspeed_recip(R cs, R bn, R bt1, R bt2, R irho) {
+// irho = 1/rho (the CUMC_FP64_FAST and mixed forms: not bit-compatible with the
+// reference); square: a2 + b2, for the range test
+template <bool NEAR, typename R>
+__device__ __forceinline__ R signalspeed_recip(R cs, R bn, R bt1, R bt2, R irho, R& square) {
     const R a2 = cs * cs;
     const R a4 = a2 * a2;
     const R b2n = (bn * bn) * irho;
@@ -263,7 +272,9 @@ __device__ __forceinline__ R signalspeed_recip(R cs, R bn, R bt1, R bt2, R irho)
     const R b2t2 = (bt2 * bt2) * irho;
     const R b2 = (b2n + b2t1) + b2t2;
     const R b4 = b2 * b2;
-    return sqrt_r(R(0.5) * ((a2 + b2) + sqrt_max0(((a4 + b4) + (R(2) * b2) * a2) - (R(4) * a2) * b2n)));
+    square = a2 + b2;
+    return root_q<NEAR>(R(0.5) *
+                        (square + root_max0_q<NEAR>(((a4 + b4) + (R(2) * b2) * a2) - (R(4) * a2) * b2n)));
 }
 
 // compute_roe (solver/definition.f90:387-392)
@@ -324,46 +335,22 @@ struct FaceSide {
 // HLL flux at a face from the left and right primitive states (8 each,
 // natural order). out receives the 7 stored components: rho, rho v, E and
 // the two tangential fields in natural (x, y, z) order.
-//
-// RECIP (the CUMC_FP64_FAST form, not bit-compatible with the reference):
-// the 21 quotients of a face share five divisors (rho of either side,
-// ggas - 1, the Roe weight sum, sR - sL), so each divisor's reciprocal is
-// formed once and the quotients become products; the values differ from the
-// reference's by a few units in the last place.
-template <int DIR, typename R, bool RECIP = false>
+template <int DIR, typename R>
 __device__ __forceinline__ void hll_flux7(const R wl[8], const R wr[8], R ggas, R out[7]) {
     constexpr int ivn = IVX + DIR;
     constexpr int ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
     using Side = FaceSide<DIR, R>;
-    R sL, sR;
-    Side L = RECIP ? Side(wl, wl[ITAU] * recip_r(wl[IRHO]) * recip_r(ggas - R(1)), typename Side::GivenEps{})
-                   : Side(wl, ggas);
-    Side Rs = RECIP ? Side(wr, wr[ITAU] * recip_r(wr[IRHO]) * recip_r(ggas - R(1)), typename Side::GivenEps{})
-                    : Side(wr, ggas);
-    if (RECIP) {
-        const R irL = recip_r(wl[IRHO]), irR = recip_r(wr[IRHO]);
-        const R csL = sqrt_r((ggas * wl[ITAU]) * irL);
-        const R csR = sqrt_r((ggas * wr[ITAU]) * irR);
-        const R cfsL = signalspeed_recip(csL, wl[ibn], wl[ibt1], wl[ibt2], irL);
-        const R cfsR = signalspeed_recip(csR, wr[ibn], wr[ibt1], wr[ibt2], irR);
-        const R sqL = sqrt_r(wl[IRHO]), sqR = sqrt_r(wr[IRHO]);
-        const R isq = recip_r(sqL + sqR);
-        const R ubar = (sqL * wl[ivn] + sqR * wr[ivn]) * isq;
-        const R cbar = (sqL * cfsL + sqR * cfsR) * isq;
-        sL = fmin(wl[ivn] - cfsL, ubar - cbar);
-        sR = fmax(wr[ivn] + cfsR, ubar + cbar);
-    } else {
-        // EOS_SOUNDSPEED (model/riemann/src/eos.f90:168)
-        const R csL = sqrt((ggas * wl[ITAU]) / wl[IRHO]);
-        const R csR = sqrt((ggas * wr[ITAU]) / wr[IRHO]);
-        const R cfsL = signalspeed(csL, wl[ibn], wl[ibt1], wl[ibt2], wl[IRHO]);
-        const R cfsR = signalspeed(csR, wr[ibn], wr[ibt1], wr[ibt2], wr[IRHO]);
-        const R sqL = sqrt(wl[IRHO]), sqR = sqrt(wr[IRHO]);
-        const R ubar = roe_avg(wl[ivn], wr[ivn], sqL, sqR);
-        const R cbar = roe_avg(cfsL, cfsR, sqL, sqR);
-        sL = fmin(wl[ivn] - cfsL, ubar - cbar);
-        sR = fmax(wr[ivn] + cfsR, ubar + cbar);
-    }
+    const Side L(wl, ggas), Rs(wr, ggas);
+    // EOS_SOUNDSPEED (model/riemann/src/eos.f90:168)
+    const R csL = sqrt((ggas * wl[ITAU]) / wl[IRHO]);
+    const R csR = sqrt((ggas * wr[ITAU]) / wr[IRHO]);
+    const R cfsL = signalspeed(csL, wl[ibn], wl[ibt1], wl[ibt2], wl[IRHO]);
+    const R cfsR = signalspeed(csR, wr[ibn], wr[ibt1], wr[ibt2], wr[IRHO]);
+    const R sqL = sqrt(wl[IRHO]), sqR = sqrt(wr[IRHO]);
+    const R ubar = roe_avg(wl[ivn], wr[ivn], sqL, sqR);
+    const R cbar = roe_avg(cfsL, cfsR, sqL, sqR);
+    const R sL = fmin(wl[ivn] - cfsL, ubar - cbar);
+    const R sR = fmax(wr[ivn] + cfsR, ubar + cbar);
     constexpr int bt_a = DIR == 0 ? IBY : IBX;  // stored tangential components
     constexpr int bt_b = DIR == 2 ? IBY : IBZ;
     const int comp[7] = {IRHO, IVX, IVY, IVZ, ITAU, bt_a, bt_b};
@@ -371,18 +358,9 @@ __device__ __forceinline__ void hll_flux7(const R wl[8], const R wr[8], R ggas, 
 #pragma unroll
         for (int c = 0; c < 7; ++c) out[c] = L.f(comp[c]);
     } else if (sL <= R(0) && sR >= R(0)) {
-        if (RECIP) {
-            const R ids = recip_r(sR - sL);
 #pragma unroll
-            for (int c = 0; c < 7; ++c) {
-                const R yl = L.f(comp[c]), yr = Rs.f(comp[c]), xl = L.u(comp[c]), xr = Rs.u(comp[c]);
-                out[c] = ((sR * yl - sL * yr) + (sL * sR) * (xr - xl)) * ids;
-            }
-        } else {
-#pragma unroll
-            for (int c = 0; c < 7; ++c)
-                out[c] = fluxhll(L.f(comp[c]), Rs.f(comp[c]), L.u(comp[c]), Rs.u(comp[c]), sL, sR);
-        }
+        for (int c = 0; c < 7; ++c)
+            out[c] = fluxhll(L.f(comp[c]), Rs.f(comp[c]), L.u(comp[c]), Rs.u(comp[c]), sL, sR);
     } else {
 #pragma unroll
         for (int c = 0; c < 7; ++c) out[c] = Rs.f(comp[c]);
@@ -484,6 +462,72 @@ __device__ __forceinline__ bool hll_flux7_rounded(const double (&wl)[8], const d
         for (int c = 0; c < 7; ++c) out[c] = Rs.f(comp[c]);
     }
     return true;
+}
+
+// The reciprocal form (CUMC_FP64_FAST and the mixed form's all-FP32 variant, not
+// bit-compatible with the reference): the 21 quotients of a face share five
+// divisors (rho of either side, ggas - 1, the Roe weight sum, sR - sL), so each
+// divisor's reciprocal is formed once and the quotients become products; the
+// values differ from the reference's by a few units in the last place.
+// NEAR (FP64): the reciprocals and roots without a branch; false where a
+// density, a pressure, gamma - 1 or a squared speed is out of the bounds
+// above, as in a cold fluid, where a field that fades squares to a subnormal.
+template <int DIR, typename R, bool NEAR>
+__device__ __forceinline__ bool hll_flux7_recip(const R (&wl)[8], const R (&wr)[8], R ggas, R (&out)[7]) {
+    constexpr int ivn = IVX + DIR;
+    constexpr int ibn = IBX + DIR, ibt1 = IBX + (DIR + 1) % 3, ibt2 = IBX + (DIR + 2) % 3;
+    constexpr int bt_a = DIR == 0 ? IBY : IBX, bt_b = DIR == 2 ? IBY : IBZ;
+    constexpr int comp[7] = {IRHO, IVX, IVY, IVZ, ITAU, bt_a, bt_b};
+    using Side = FaceSide<DIR, R>;
+    const R gm1 = ggas - R(1);
+    if constexpr (NEAR)
+        if (range_max(wl[IRHO],
+                      range_max(wr[IRHO], range_max(wl[ITAU], range_max(wr[ITAU], range_max(gm1, 0u))))) >= RANGE_SPAN)
+            return false;
+    const R irL = recip_q<NEAR>(wl[IRHO]), irR = recip_q<NEAR>(wr[IRHO]), ig = recip_q<NEAR>(gm1);
+    const Side L(wl, wl[ITAU] * irL * ig, typename Side::GivenEps{});
+    const Side Rs(wr, wr[ITAU] * irR * ig, typename Side::GivenEps{});
+    R squareL, squareR;
+    const R csL = root_q<NEAR>((ggas * wl[ITAU]) * irL);
+    const R csR = root_q<NEAR>((ggas * wr[ITAU]) * irR);
+    const R cfsL = signalspeed_recip<NEAR>(csL, wl[ibn], wl[ibt1], wl[ibt2], irL, squareL);
+    const R cfsR = signalspeed_recip<NEAR>(csR, wr[ibn], wr[ibt1], wr[ibt2], irR, squareR);
+    if constexpr (NEAR)
+        if (max(hi_word(squareL), hi_word(squareR)) >= SQUARE_MAX) return false;
+    const R sqL = root_q<NEAR>(wl[IRHO]), sqR = root_q<NEAR>(wr[IRHO]);
+    const R isq = recip_q<NEAR>(sqL + sqR);
+    const R ubar = (sqL * wl[ivn] + sqR * wr[ivn]) * isq;
+    const R cbar = (sqL * cfsL + sqR * cfsR) * isq;
+    const R sL = fmin(wl[ivn] - cfsL, ubar - cbar);
+    const R sR = fmax(wr[ivn] + cfsR, ubar + cbar);
+    if (sL >= R(0)) {
+#pragma unroll
+        for (int c = 0; c < 7; ++c) out[c] = L.f(comp[c]);
+    } else if (sL <= R(0) && sR >= R(0)) {
+        // (at least a Roe-weighted sound speed, 2^-400, and less than 2^1000 unless
+        // a velocity makes every product below infinite as well)
+        const R ids = recip_q<NEAR>(sR - sL);
+#pragma unroll
+        for (int c = 0; c < 7; ++c) {
+            const R yl = L.f(comp[c]), yr = Rs.f(comp[c]), xl = L.u(comp[c]), xr = Rs.u(comp[c]);
+            out[c] = ((sR * yl - sL * yr) + (sL * sR) * (xr - xl)) * ids;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 7; ++c) out[c] = Rs.f(comp[c]);
+    }
+    return true;
+}
+// its form with the IEEE operations, out of line
+template <int DIR>
+__device__ __noinline__ void hll_flux7_recip_ieee(const double* w, double ggas, double* out) {
+    double wl[8], wr[8], fx[7];
+    for (int q = 0; q < 8; ++q) {
+        wl[q] = w[q];
+        wr[q] = w[8 + q];
+    }
+    hll_flux7_recip<DIR, double, false>(wl, wr, ggas, fx);
+    for (int q = 0; q < 7; ++q) out[q] = fx[q];
 }
 
 // ---------------------------------------------------------------------------
@@ -591,7 +635,7 @@ __device__ __forceinline__ void geom_ct(const Tabs& T, int j, int k, int l, CTf&
 // ---------------------------------------------------------------------------
 // HLL of the mixed form (float states). The wave speeds and the two stored
 // tangential-field components are formed in FP32, in the reciprocal form of
-// hll_flux7 (five divisors, each reciprocal formed once); the five hydro
+// hll_flux7_recip (five divisors, each reciprocal formed once); the five hydro
 // components (rho, rho v, E) take their side fluxes, conserved values and HLL
 // combination in FP64 from the FP32 states, with each side's internal energy,
 // E, B^2/2 and v.B in FP64. Measured on Orszag-Tang 256^3 to t = 0.5, the
@@ -640,20 +684,6 @@ __device__ __forceinline__ SideScalars side_scalars64(const float (&w)[8], float
     return {rho * (e + 0.5 * vsq) + 0.5 * bsq, 0.5 * bsq, (bx * vx + by * vy) + bz * vz};
 }
 
-// signalspeed_recip in FP32 with the roots' form chosen
-template <bool ROUNDED>
-__device__ __forceinline__ float signalspeed_q(float cs, float bn, float bt1, float bt2, float irho) {
-    const float a2 = cs * cs;
-    const float a4 = a2 * a2;
-    const float b2n = (bn * bn) * irho;
-    const float b2t1 = (bt1 * bt1) * irho;
-    const float b2t2 = (bt2 * bt2) * irho;
-    const float b2 = (b2n + b2t1) + b2t2;
-    const float b4 = b2 * b2;
-    return root_q<ROUNDED>(
-        0.5f * ((a2 + b2) + root_max0_q<ROUNDED>(((a4 + b4) + (2.0f * b2) * a2) - (4.0f * a2) * b2n)));
-}
-
 // ROUNDED: the five FP32 reciprocals and eight roots without their range
 // branches; false (nothing computed) where a density leaves [2^-60, 2^60) or
 // gamma p/rho leaves [2^-38, 2^45)
@@ -672,8 +702,9 @@ __device__ __forceinline__ bool hll_flux7_mixed_form(const float (&wl)[8], const
             return false;
         const float csL = root_q<ROUNDED>(xL);
         const float csR = root_q<ROUNDED>(xR);
-        const float cfsL = signalspeed_q<ROUNDED>(csL, wl[ibn], wl[ibt1], wl[ibt2], irL);
-        const float cfsR = signalspeed_q<ROUNDED>(csR, wr[ibn], wr[ibt1], wr[ibt2], irR);
+        float squareL, squareR;
+        const float cfsL = signalspeed_recip<ROUNDED>(csL, wl[ibn], wl[ibt1], wl[ibt2], irL, squareL);
+        const float cfsR = signalspeed_recip<ROUNDED>(csR, wr[ibn], wr[ibt1], wr[ibt2], irR, squareR);
         const float sqL = root_q<ROUNDED>(wl[IRHO]), sqR = root_q<ROUNDED>(wr[IRHO]);
         const float isq = recip_q<ROUNDED>(sqL + sqR);
         const float ubar = (sqL * wl[ivn] + sqR * wr[ivn]) * isq;
@@ -747,25 +778,27 @@ __device__ __forceinline__ void hll_flux7_mixed(const float (&wl)[8], const floa
 }
 
 
-// the sweeps' HLL solve: hll_flux7 in FP64 (RECIP: the CUMC_FP64_FAST form).
-// For the mixed form's float states, RECIP selects the all-FP32 reciprocal
-// form of hll_flux7 (faster; density 1.06e-5 from the FP64 run at t_end above)
+// the sweeps' HLL solve: hll_flux7's values in FP64 (RECIP: the CUMC_FP64_FAST
+// form). For the mixed form's float states, RECIP selects the all-FP32
+// reciprocal form (faster; density 1.06e-5 from the FP64 run at t_end above)
 // and its absence hll_flux7_mixed (the default).
 template <int DIR, typename R, bool RECIP>
 __device__ __forceinline__ void sweep_hll(const R (&wl)[8], const R (&wr)[8], R ggas, R (&fx)[7]) {
     if constexpr (sizeof(R) == 4) {
-        if constexpr (RECIP) hll_flux7<DIR, R, true>(wl, wr, ggas, fx);
+        if constexpr (RECIP) hll_flux7_recip<DIR, R, false>(wl, wr, ggas, fx);
         else hll_flux7_mixed<DIR>(wl, wr, ggas, fx);
-    } else if constexpr (RECIP) {
-        hll_flux7<DIR, R, true>(wl, wr, ggas, fx);
-    } else if (!hll_flux7_rounded<DIR>(wl, wr, ggas, fx)) {
+    } else {
+        const bool done = RECIP ? hll_flux7_recip<DIR, double, true>(wl, wr, ggas, fx)
+                                : hll_flux7_rounded<DIR>(wl, wr, ggas, fx);
+        if (done) return;
         double w[16], f[7];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             w[q] = wl[q];
             w[8 + q] = wr[q];
         }
-        hll_flux7_ieee<DIR>(w, ggas, f);
+        if constexpr (RECIP) hll_flux7_recip_ieee<DIR>(w, ggas, f);
+        else hll_flux7_ieee<DIR>(w, ggas, f);
 #pragma unroll
         for (int q = 0; q < 7; ++q) fx[q] = f[q];
     }

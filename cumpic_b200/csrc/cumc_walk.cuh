@@ -356,7 +356,7 @@ constexpr int WK_SLOTS = 6;  // slots of the fused walkers (cumc_fused.cuh): a r
 // reconstructed states, left in out and right in out_r (field order of the
 // sweep, at the face's left cell), for the adjoint's HLL transpose.
 // c_lo, c_cnt, c_step: the columns walked (WalkCol; c_cnt < 0 for all)
-// RECIP: the HLL solve's quotients as products with reciprocals (hll_flux7)
+// RECIP: the HLL solve's quotients as products with reciprocals (hll_flux7_recip)
 template <int DIR, int RECON, typename R, bool STATES = false, bool RECIP = false>
 __global__ void __launch_bounds__(WK_THREADS, CUMC_WALK_MINB) k_sweep_walk_sm(Box b, Tabs T, PrimT<R> pr, R ggas, FaceFluxT<R> out,
                                                              int seg, FaceFluxT<R> out_r, int c_lo, int c_cnt, int c_step) {
