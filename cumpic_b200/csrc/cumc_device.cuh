@@ -685,8 +685,9 @@ __device__ __forceinline__ SideScalars side_scalars64(const float (&w)[8], float
 }
 
 // ROUNDED: the five FP32 reciprocals and eight roots without their range
-// branches; false (nothing computed) where a density leaves [2^-60, 2^60) or
-// gamma p/rho leaves [2^-38, 2^45)
+// branches; false (nothing computed) where a density leaves [2^-60, 2^60), gamma
+// p/rho [2^-38, 2^45), or a2 + b2 is not below 2^49 (its square then exceeds the
+// roots' 2^100, or is infinite or NaN)
 template <int DIR, bool ROUNDED>
 __device__ __forceinline__ bool hll_flux7_mixed_form(const float (&wl)[8], const float (&wr)[8], float ggas,
                                                      float (&out)[7]) {
@@ -705,6 +706,7 @@ __device__ __forceinline__ bool hll_flux7_mixed_form(const float (&wl)[8], const
         float squareL, squareR;
         const float cfsL = signalspeed_recip<ROUNDED>(csL, wl[ibn], wl[ibt1], wl[ibt2], irL, squareL);
         const float cfsR = signalspeed_recip<ROUNDED>(csR, wr[ibn], wr[ibt1], wr[ibt2], irR, squareR);
+        if (ROUNDED && max(__float_as_uint(squareL), __float_as_uint(squareR)) >= (127u + 49u) << 23) return false;
         const float sqL = root_q<ROUNDED>(wl[IRHO]), sqR = root_q<ROUNDED>(wr[IRHO]);
         const float isq = recip_q<ROUNDED>(sqL + sqR);
         const float ubar = (sqL * wl[ivn] + sqR * wr[ivn]) * isq;

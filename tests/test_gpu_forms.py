@@ -275,6 +275,13 @@ def test_recip_solve_keeps_non_finite_speeds(lib64):
         assert not bad.any(), (d, w[bad.any(axis=1)][0], f[bad.any(axis=1)][0], ref[bad.any(axis=1)][0])
 
 
+def test_hll_mixed_is_its_plain_form(lib32):
+    w = edge_states(np.float32, SPECIAL32, SCALE32, 6)
+    for d, (f, ref, _) in enumerate(_hll(lib32.hll_mixed, w, ctypes.c_float(GGAS), np.float32)):
+        bad = ~_same(f, ref).all(axis=1)
+        assert not bad.any(), (d, bad.sum(), w[bad][0], f[bad][0], ref[bad][0])
+
+
 def test_recip_run_with_faint_fields_and_no_pressure():
     """A cold fluid at rest in a field of 1e-78: B^2/rho squared is subnormal
     (2e-311, known to 2.5e-13 of itself). Against the FP64 oracle at the
