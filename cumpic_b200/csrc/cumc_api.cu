@@ -78,6 +78,7 @@ struct cumc_ctx {
     cudaGraphExec_t rk_exec = nullptr;  // the launches of one cumc_rungekutta (rk_step_host)
     long long rk_launches = 0;
     int rk_calls = 0;
+    bool rk_plain = false;  // it failed: the step is launched kernel by kernel
     cudaGraphExec_t graph_exec = nullptr;
     double graph_t_end = 0.0;
     long long graph_launches_per_step = 0;
@@ -802,39 +803,41 @@ void rk_step_dt(cumc_ctx* c, const Box& b) {
     c->fuse_dt = false;
 }
 
+// one rk_step_dt recorded into c->rk_exec; the context's stream keeps running as
+// before if that fails
+cudaError_t capture_rk_step(cumc_ctx* c) {
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    const long long before = c->launches;
+    c->fork = true;
+    rk_step_dt(c, c->box);
+    c->fork = false;
+    c->rk_launches = c->launches - before;
+    c->launches = before;
+    e = cudaStreamEndCapture(c->stream, &g);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&c->rk_exec, g, 0);
+    if (e != cudaSuccess) c->rk_exec = nullptr;
+    if (g) cudaGraphDestroy(g);
+    return e;
+}
+
 // The step of cumc_rungekutta. Its launches are the same every call (dt and the
 // state stay in their places on the device), so from the second call on they
 // go as one graph: on small boxes the host's launches took longer than the
-// kernels. Launched one by one under per-kernel timing and while the caller
-// captures the stream.
-int rk_step_host(cumc_ctx* c) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CUMC_CHECK(cudaStreamIsCapturing(c->stream, &cap));
-    const bool plain = c->prof_on || cap != cudaStreamCaptureStatusNone || (!c->rk_exec && c->rk_calls++ == 0);
-    if (!plain && !c->rk_exec) {
-        cudaGraph_t g;
-        const long long before = c->launches;
-        CUMC_CHECK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        c->fork = true;
-        rk_step_dt(c, c->box);
-        c->fork = false;
-        c->rk_launches = c->launches - before;
-        c->launches = before;
-        CUMC_CHECK(cudaStreamEndCapture(c->stream, &g));
-        const cudaError_t e = cudaGraphInstantiate(&c->rk_exec, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) {
-            c->rk_exec = nullptr;
-            return cuda_fail(c, e, "cudaGraphInstantiate");
+// kernels. Launched one by one under per-kernel timing, while the caller
+// captures the stream, and where the graph cannot be made or launched.
+void rk_step_host(cumc_ctx* c, bool captured) {
+    if (!c->prof_on && !captured && !c->rk_plain && (c->rk_exec || c->rk_calls++ > 0)) {
+        if ((c->rk_exec || capture_rk_step(c) == cudaSuccess) &&
+            cudaGraphLaunch(c->rk_exec, c->stream) == cudaSuccess) {
+            c->launches += c->rk_launches;
+            return;
         }
+        cudaGetLastError();  // no memory for a graph, say (an error that lasts shows in the launches below)
+        c->rk_plain = true;
     }
-    if (plain) {
-        rk_step_dt(c, c->box);
-    } else {
-        CUMC_CHECK(cudaGraphLaunch(c->rk_exec, c->stream));
-        c->launches += c->rk_launches;
-    }
-    return CUMC_OK;
+    rk_step_dt(c, c->box);
 }
 
 void finddt_launch(cumc_ctx* c, const Box& b) {
@@ -1460,11 +1463,18 @@ int cumc_rungekutta(cumc_ctx* c, double dt) {
     if (c->next_stage != 1) return c->fail(CUMC_ERR_STATE, "cumc_rk_stage left a step unfinished");
     if (!(dt >= 0.0 && std::isfinite(dt))) return c->fail(CUMC_ERR_ARG, "dt must be finite and non-negative");
     // stage 3 forms the next step's CFL dt, which cumc_finddt then returns
-    // without a pass over the state (the same expression, so the same bits)
+    // without a pass over the state (the same expression, so the same bits):
+    // valid once the step has been issued. A step that a caller captures runs
+    // later or never, and leaves dtmin and the mark as they are.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUMC_CHECK(cudaStreamIsCapturing(c->stream, &cap));
+    const bool captured = cap != cudaStreamCaptureStatusNone;
+    if (!captured) c->dt_valid = false;
     launch(c, -1, 1, 1, k_set_dt, make_clock(c), dt);
-    if ((rc = rk_step_host(c)) != CUMC_OK) return rc;
-    c->dt_valid = true;
-    return sync_status(c);
+    rk_step_host(c, captured);
+    if ((rc = sync_status(c)) != CUMC_OK) return rc;
+    if (!captured) c->dt_valid = true;
+    return CUMC_OK;
 }
 
 int cumc_rk_stage_part(cumc_ctx* c, int stage, double dt, int part) {
