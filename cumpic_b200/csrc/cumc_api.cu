@@ -695,7 +695,7 @@ void fused_stage(cumc_ctx* c, const Box& b, int stage, const Prim& pr, double* c
 // ghost plane, 2 the rest (see fused_stage); the unfused forms run the whole
 // stage at part 0 and 2 and nothing at part 1
 void run_stage(cumc_ctx* c, const Box& b, int stage, int part = 0) {
-    if (stage > 0) c->lrk_valid = false;
+    if (stage > 0) c->lrk_valid = false;  // (a step that replays a graph does not come here)
     static const char* const names[4] = {"cumc spatial", "cumc rk stage 1", "cumc rk stage 2", "cumc rk stage 3"};
     const NvtxRange range(names[stage]);
     if (c->mixed) {
@@ -1470,6 +1470,7 @@ int cumc_rungekutta(cumc_ctx* c, double dt) {
     CUMC_CHECK(cudaStreamIsCapturing(c->stream, &cap));
     const bool captured = cap != cudaStreamCaptureStatusNone;
     if (!captured) c->dt_valid = false;
+    c->lrk_valid = false;
     launch(c, -1, 1, 1, k_set_dt, make_clock(c), dt);
     rk_step_host(c, captured);
     if ((rc = sync_status(c)) != CUMC_OK) return rc;
@@ -1593,6 +1594,7 @@ int cumc_advance(cumc_ctx* c, int nsteps, double t_end, double* t_inout, int* st
     if (c->exchange) return c->fail(CUMC_ERR_STATE, "a slab with CUMC_BC_EXCHANGE faces steps by cumc_rk_stage and the halo exchange");
     if (c->next_stage != 1) return c->fail(CUMC_ERR_STATE, "cumc_rk_stage left a step unfinished");
     if (nsteps < 0 || !t_inout) return c->fail(CUMC_ERR_ARG, "nsteps must be >= 0 and t_inout non-null");
+    if (nsteps > 0) c->lrk_valid = false;
     launch(c, -1, 1, 1, k_set_scalar, c->scal + 1, *t_inout);
     CUMC_CHECK(cudaMemsetAsync(c->ints, 0, 2 * sizeof(int), c->stream));
     if (nsteps > 0) finddt_launch(c, c->box);  // dt of the first iteration; stage 3 gives the rest

@@ -101,6 +101,23 @@ def test_dt_after_a_capture_that_never_ran():
     assert g.finddt() == o.finddt()
 
 
+def test_l_rk_is_stale_after_a_step():
+    """cumc_download_lrk refuses an l_rk that a step has outdated, also where
+    the step's launches come from a graph"""
+    from cumpic_b200.solver import CUMC3D
+    g = CUMC3D(P.orszag_tang(10, ny=9, nz=8))
+    g.upload()
+    g.initial_update()
+    out = np.empty(g.shape + (8,))
+    ptr = out.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+    for move in (lambda: g.rungekutta(g.finddt()), lambda: g.advance(1)):
+        for _ in range(6):
+            move()
+            assert g._lib.cumc_download_lrk(g._h, ptr) == N.CUMC_ERR_STATE
+            g.spatial()
+            assert g._lib.cumc_download_lrk(g._h, ptr) == N.CUMC_OK
+
+
 @pytest.mark.parametrize("coordinate", [N.CYLINDRICAL, N.SPHERICAL], ids=["cylindrical", "spherical"])
 @pytest.mark.parametrize("scale,amp", [(1e-61, 1.0), (1e-60, 1.0), (1e60, 1.0), (1e61, 1.0), (1.0, 1e-155),
                                        (1.0, 1e-290), (1.0, 1e-318)])
