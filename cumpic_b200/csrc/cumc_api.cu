@@ -823,12 +823,20 @@ cudaError_t capture_rk_step(cumc_ctx* c) {
 }
 
 // The step of cumc_rungekutta. Its launches are the same every call (dt and the
-// state stay in their places on the device), so from the second call on they
-// go as one graph: on small boxes the host's launches took longer than the
+// state stay in their places on the device), so from the RK_GRAPH_CALL-th call on
+// they go as one graph: on small boxes the host's launches took longer than the
 // kernels. Launched one by one under per-kernel timing, while the caller
 // captures the stream, and where the graph cannot be made or launched.
+// Capturing and instantiating costs 340-360 us more than a step launched one by
+// one, and a replay saves 45-85 (finddt and step, synchronised: 512x4x4 tube 205
+// us a step, 546 with the capture, then 141; 64^3 415, 772, 372; 90x26x75 360,
+// 721, 305; 128^3 2048, 2360, 1962). So six steps are run first, about what the
+// capture costs, and it comes with the seventh: a context that takes fewer
+// never pays for it. With the capture in the second call a context of two steps
+// took 1.8 times as long.
+constexpr int RK_GRAPH_CALL = 7;
 void rk_step_host(cumc_ctx* c, bool captured) {
-    if (!c->prof_on && !captured && !c->rk_plain && (c->rk_exec || c->rk_calls++ > 0)) {
+    if (!c->prof_on && !captured && !c->rk_plain && (c->rk_exec || ++c->rk_calls >= RK_GRAPH_CALL)) {
         if ((c->rk_exec || capture_rk_step(c) == cudaSuccess) &&
             cudaGraphLaunch(c->rk_exec, c->stream) == cudaSuccess) {
             c->launches += c->rk_launches;

@@ -111,7 +111,7 @@ def test_l_rk_is_stale_after_a_step():
     out = np.empty(g.shape + (8,))
     ptr = out.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
     for move in (lambda: g.rungekutta(g.finddt()), lambda: g.advance(1)):
-        for _ in range(6):
+        for _ in range(10):
             move()
             assert g._lib.cumc_download_lrk(g._h, ptr) == N.CUMC_ERR_STATE
             g.spatial()
