@@ -468,14 +468,13 @@ struct FaceAdj {
 // normal-field adjoint of the face to lambf. Four 128-thread blocks per SM
 // (128 registers, 40 bytes spilled); 268 -> 178 us a launch at 128^3 with the two
 // sides one after the other (hll_adj), FP64 pipe 57 % busy.
-// FROM_STATES: fa already holds the forward states (the forward sweep's
-// STATES form, one reconstruction per cell); each face reads its two states
-// and overwrites them with their adjoints. Otherwise the face reconstructs
-// its two cells itself.
+// fa holds the forward states (the forward sweep's STATES form, one
+// reconstruction per cell: vp_out of cell c, vm_out of cell c+1); each face reads
+// its two states and overwrites them with their adjoints.
 #ifndef CUMC_ADJ_MINB
 #define CUMC_ADJ_MINB 4
 #endif
-template <int COORD, int DIR, int RECON, bool FROM_STATES = false>
+template <int COORD, int DIR>
 __global__ void __launch_bounds__(128, CUMC_ADJ_MINB) k_adj_hll(Box b, Tabs T, Prim pr, double ggas, AdjStage a, FaceAdj fa,
                                                 double* lambf) {
     const int n0 = (DIR == 0 ? b.nx : b.nx + 1) + 1;
@@ -547,40 +546,13 @@ __global__ void __launch_bounds__(128, CUMC_ADJ_MINB) k_adj_hll(Box b, Tabs T, P
 
     constexpr int bt_a = DIR == 0 ? 1 : 0;
     constexpr int bt_b = DIR == 2 ? 1 : 2;
-    const double* src[7] = {pr.w[0], pr.w[1], pr.w[2], pr.w[3], pr.w[4], pr.bc[bt_a], pr.bc[bt_b]};
     const int slot[7] = {IRHO, IVX, IVY, IVZ, ITAU, IBX + bt_a, IBX + bt_b};
 
-    // forward states (the forward sweep's values: vp_out of cell c, vm_out of cell c+1)
     double wl[8], wr[8];
 #pragma unroll
     for (int v = 0; v < 7; ++v) {
-        if (FROM_STATES) {
-            wl[slot[v]] = fa.l[v][base];
-            wr[slot[v]] = fa.r[v][base];
-            continue;
-        }
-        const double* q = src[v] + base;
-        double cv[6];
-#pragma unroll
-        for (int m = 0; m < 6; ++m) cv[m] = q[(m - 2) * s];  // cells c-2..c+3
-        double vm, vp;
-        if (RECON == 4) {
-            const double dmm = ppm_slope(cv[0], cv[1], cv[2], A.s0[c - 1], A.s1[c - 1]);
-            const double dmc = ppm_slope(cv[1], cv[2], cv[3], A.s0[c], A.s1[c]);
-            const double dmp = ppm_slope(cv[2], cv[3], cv[4], A.s0[c + 1], A.s1[c + 1]);
-            const double dmq = ppm_slope(cv[3], cv[4], cv[5], A.s0[c + 2], A.s1[c + 2]);
-            const double V0 = ppm_face(cv[1], cv[2], dmm, dmc, A.a0[c - 1], A.a1[c - 1], A.a2[c - 1], A.a3[c - 1]);
-            const double V1 = ppm_face(cv[2], cv[3], dmc, dmp, A.a0[c], A.a1[c], A.a2[c], A.a3[c]);
-            const double V2 = ppm_face(cv[3], cv[4], dmp, dmq, A.a0[c + 1], A.a1[c + 1], A.a2[c + 1], A.a3[c + 1]);
-            double vm0, vp1;
-            ppm_fix(cv[2], V0, V1, vm0, vp);
-            ppm_fix(cv[3], V1, V2, vm, vp1);
-        } else {
-            vp = cv[2] + 0.5 * tvd_slope(cv[1], cv[2], cv[3], A.tcf[c], A.tcb[c]);
-            vm = cv[3] - 0.5 * tvd_slope(cv[2], cv[3], cv[4], A.tcf[c + 1], A.tcb[c + 1]);
-        }
-        wl[slot[v]] = vp;
-        wr[slot[v]] = vm;
+        wl[slot[v]] = fa.l[v][base];
+        wr[slot[v]] = fa.r[v][base];
     }
     const double bn = pr.bf[DIR][base];
     wl[IBX + DIR] = bn;

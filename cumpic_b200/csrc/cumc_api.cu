@@ -255,11 +255,11 @@ void sweep_xpair(cumc_ctx* c, const Box& b, const Prim& pr, const FaceFlux& out,
                     l_step);
     };
     if (c->fast)
-        vec ? go(ppm ? k_sweep_xpair<4, double, true, true> : k_sweep_xpair<1, double, true, true>)
-            : go(ppm ? k_sweep_xpair<4, double, true, false> : k_sweep_xpair<1, double, true, false>);
+        vec ? go(ppm ? k_sweep_xpair<4, true, true> : k_sweep_xpair<1, true, true>)
+            : go(ppm ? k_sweep_xpair<4, true, false> : k_sweep_xpair<1, true, false>);
     else
-        vec ? go(ppm ? k_sweep_xpair<4, double, false, true> : k_sweep_xpair<1, double, false, true>)
-            : go(ppm ? k_sweep_xpair<4, double, false, false> : k_sweep_xpair<1, double, false, false>);
+        vec ? go(ppm ? k_sweep_xpair<4, false, true> : k_sweep_xpair<1, false, true>)
+            : go(ppm ? k_sweep_xpair<4, false, false> : k_sweep_xpair<1, false, false>);
 }
 
 // l_lo, l_cnt, l_step: the z planes whose x rows (DIR 0) or y columns (DIR 1) the
@@ -268,7 +268,7 @@ template <int DIR>
 void sweep(cumc_ctx* c, const Box& b, const Prim& pr, int l_lo = 0, int l_cnt = -1, int l_step = 1) {
     FaceFlux out;
     for (int q = 0; q < 7; ++q) out.f[q] = c->F[DIR][q];
-    // default: one lane per cell along x, the shared-memory-window walker
+    // default: two cells a lane along x, the shared-memory-window walker
     // along y and z
     // modes 0 and 9 come here only for SPATIAL alone (stage 0) and take the
     // unfused default's kernels
@@ -433,23 +433,16 @@ UtopArgs utop_args(cumc_ctx* c, double* const* u, const PrimBufs& p) {
     return a;
 }
 
-void utop_into(cumc_ctx* c, const Box& b, double* const* u, const PrimBufs& p, bool from_cons) {
-    const UtopArgs a = utop_args(c, u, p);
+// initial_update's conversions
+void utop(cumc_ctx* c, const Box& b, double* const* u) {
+    const UtopArgs a = utop_args(c, u, PrimBufs{c->w, c->bc, c->eps});
     const long long n = (long long)(b.nx + 1) * (b.ny + 1) * (b.nz + 1);
-#define CUMC_UTOP(M)                                                                         \
-    if (from_cons) launch(c, CUMC_K_UTOP, n, 256, k_utop<M, true>, b, a);                    \
-    else launch(c, CUMC_K_UTOP, n, 256, k_utop<M, false>, b, a);
     switch (c->model) {
-        case CUMC_MODEL_NONE: CUMC_UTOP(0) break;
-        case CUMC_MODEL_RIEMANN: CUMC_UTOP(1) break;
-        case CUMC_MODEL_TORUS_SPH: CUMC_UTOP(2) break;
-        default: CUMC_UTOP(3) break;
+        case CUMC_MODEL_NONE: launch(c, CUMC_K_UTOP, n, 256, k_utop<0>, b, a); break;
+        case CUMC_MODEL_RIEMANN: launch(c, CUMC_K_UTOP, n, 256, k_utop<1>, b, a); break;
+        case CUMC_MODEL_TORUS_SPH: launch(c, CUMC_K_UTOP, n, 256, k_utop<2>, b, a); break;
+        default: launch(c, CUMC_K_UTOP, n, 256, k_utop<3>, b, a); break;
     }
-#undef CUMC_UTOP
-}
-
-void utop(cumc_ctx* c, const Box& b, double* const* u, bool from_cons) {
-    utop_into(c, b, u, PrimBufs{c->w, c->bc, c->eps}, from_cons);
 }
 
 BoundArgs bound_args(cumc_ctx* c, double* const* u, const PrimBufs& p) {
@@ -1439,7 +1432,7 @@ int cumc_initial_update(cumc_ctx* c) {
         c->ready = true;
         return sync_status(c);
     }
-    utop(c, c->box, c->U[c->cur], false);
+    utop(c, c->box, c->U[c->cur]);
     boundary(c, c->box, c->U[c->cur]);
     c->ready = true;
     c->next_stage = 1;
@@ -1837,15 +1830,15 @@ void adj_sweeps(cumc_ctx* c, const Box& b, const Prim& pr, const AdjStage& st, c
     };
     // x: pass A per face, pass B one lane per cell and field
     launch(c, -1, xwarp_threads(b), 128, k_sweep_xwarp<RECON, double, true>, b, c->tabs, pr, c->ggas, sl, sr, 0, -1);
-    launch(c, -1, fx, 128, k_adj_hll<COORD, 0, RECON, true>, b, c->tabs, pr, c->ggas, st, fa, lbf[0]);
+    launch(c, -1, fx, 128, k_adj_hll<COORD, 0>, b, c->tabs, pr, c->ggas, st, fa, lbf[0]);
     launch_grid(c, -1, dim3((unsigned)((recon_x_warps(b) * 32 + 127) / 128), 7), 128, 0, k_adj_recon_x<RECON>, b,
                 c->tabs, pr, fa, lp);
     // y, z: pass A per face, pass B one thread per (column, field)
     states(std::integral_constant<int, 1>{});
-    launch(c, -1, fy, 128, k_adj_hll<COORD, 1, RECON, true>, b, c->tabs, pr, c->ggas, st, fa, lbf[1]);
+    launch(c, -1, fy, 128, k_adj_hll<COORD, 1>, b, c->tabs, pr, c->ggas, st, fa, lbf[1]);
     recon_col<1, RECON>(c, b, pr, fa, lp);
     states(std::integral_constant<int, 2>{});
-    launch(c, -1, fz, 128, k_adj_hll<COORD, 2, RECON, true>, b, c->tabs, pr, c->ggas, st, fa, lbf[2]);
+    launch(c, -1, fz, 128, k_adj_hll<COORD, 2>, b, c->tabs, pr, c->ggas, st, fa, lbf[2]);
     recon_col<2, RECON>(c, b, pr, fa, lp);
 }
 
@@ -1959,7 +1952,7 @@ int adjoint_run(cumc_ctx* c, int N, int K, int obj, const double* weights, const
     zero_lp();
 
     // ---- forward pass with checkpoints (initial_update, then N steps) ------
-    utop(c, b, c->U[c->cur], false);
+    utop(c, b, c->U[c->cur]);
     boundary(c, b, c->U[c->cur]);
     std::vector<double> dts((size_t)N);
     const int last0 = (nck - 1) * K;  // the last segment is taped now, not recomputed

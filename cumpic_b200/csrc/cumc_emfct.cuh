@@ -5,7 +5,7 @@
 // fields, solver/rungekutta.f90:41-51,75-85,109-119).
 //
 // k_emf writes the three edge-EMF arrays and k_ct reads them back at six
-// neighbouring edges a face triple. Here a block owns a tile of 32 x 8 face
+// neighbouring edges a face triple. Here a block owns a tile of 32 x 4 face
 // triples (x fastest) and marches in z over a segment of planes. Per plane
 // it forms, in shared memory, the cell EMFs E = -v x B of the cells the
 // plane's edges average, then the edge EMFs of the tile and of the halo row

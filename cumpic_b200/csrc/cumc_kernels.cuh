@@ -393,14 +393,14 @@ __global__ void __launch_bounds__(256, 8) k_ct(Box b, Tabs T, CombineArgs a) {
 }
 
 // ----------------------------------------------------------------------------
-// k_utop: on (0:n)^3, FROMUTORVE (solver/fromrvetou.f90:75-127, UtoP_MHD
-// solver/utop.f90:33-68), CUSTOM_CHECKRHO (interior), FROMRVETOU's P_to_U
-// (solver/ptou.f90:33-66) and UPDATE's pressure on the interior
-// (solver/update.f90:27-35). FROM_CONS=false is initial_update: the
-// primitives come from the uploaded model instead of from cons.
+// k_utop: initial_update's conversions on (0:n)^3, from the uploaded primitives:
+// CUSTOM_CHECKRHO (interior), FROMRVETOU's P_to_U (solver/ptou.f90:33-66) and
+// UPDATE's pressure on the interior (solver/update.f90:27-35). In a stage they
+// follow FROMUTORVE (solver/fromrvetou.f90:75-127, UtoP_MHD
+// solver/utop.f90:33-68) in the combine.
 // ----------------------------------------------------------------------------
 struct UtopArgs {
-    double* u[8];       // cons: read, hydro part rewritten
+    double* u[8];       // cons: hydro part rewritten, face fields read
     double* w[5];       // rho, vx, vy, vz, p
     double* bc[3];
     double* eps;
@@ -532,19 +532,14 @@ __device__ __forceinline__ void utop_point(const UtopArgs& a, int i, bool interi
     }
 }
 
-template <int MODEL, bool FROM_CONS>
+template <int MODEL>
 __global__ void __launch_bounds__(256) k_utop(Box b, UtopArgs a) {
     int j, k, l, i;
     if (!box1_index(b, j, k, l, i)) return;
     const bool interior = j >= 1 && k >= 1 && l >= 1;
     double bx, by, bz;
     bcell_point(b, a, i, interior, bx, by, bz);
-    double uh[5];
-    if (FROM_CONS) {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) uh[q] = a.u[q][i];
-    }
-    utop_point<MODEL, FROM_CONS>(a, i, interior, uh, bx, by, bz);
+    utop_point<MODEL, false>(a, i, interior, nullptr, bx, by, bz);
 }
 
 // What a stage leaves behind. Inside a whole step (a.lean; not between

@@ -57,15 +57,15 @@ struct WalkGeom {
 };
 
 // Segments of a walk along DIR over `ncols` columns. Equal blocks run in
-// rounds of the WK_RESIDENT blocks a SM that fit (96 registers and 21.5 KB of
-// shared memory a 64-thread block), and a segment costs its faces plus a
+// rounds of the WK_RESIDENT blocks a SM that fit (96 registers and 17.5 KB of
+// shared memory a 64-thread block with PPM, 14 KB with TVD), and a segment costs its faces plus a
 // prologue (three slopes, two interface values and a fix a field, and a
 // memory latency: about one and a half faces), so the count is taken that
 // makes rounds x (faces + 1.5) least. Against about 64 faces, halved down to
 // 8 while the grid gave fewer than 32 warps a SM: 64^3 0.036 -> 0.029 ms a
 // walk, the 90x26x75 torus 0.029 -> 0.023, a 512x4x4 tube 0.021 -> 0.013; 256^3
 // unchanged (0.90).
-constexpr int WK_RESIDENT = 10, WK_SEG_MAX = 64;  // (64 faces: 3 KB of weights a block)
+constexpr int WK_RESIDENT = 10, WK_SEG_MAX = 64;  // (64 faces: 1.5 KB of FP32 weights a mixed block)
 template <int DIR>
 inline int walk_segment_for(const Box& b, long long ncols, int sm_count, int* nseg) {
     const int faces = WalkGeom<DIR>::nd(b) + 1;
@@ -552,29 +552,20 @@ inline long long xwarp_threads(const Box& b, int l_cnt = -1) {
 // costs nothing but its five faces that straddle the row's end, which are
 // skipped. The pair's states wait in shared memory between the reconstruction
 // and the two solves (one body, run twice), which keeps the registers to the
-// walkers' 96. VEC: with SX even a pair starts on a 16-byte boundary (8 bytes
-// in FP32) and moves as one vector.
+// walkers' 96. VEC: with SX even a pair starts on a 16-byte boundary and moves as
+// one vector.
 // ---------------------------------------------------------------------------
 constexpr int XP_FACES = 58, XP_THREADS = 128;
 #ifndef CUMC_XPAIR_MINB
 #define CUMC_XPAIR_MINB 5
 #endif
-template <typename R>
-struct Pair {
-    R a, b;
-};
-template <bool VEC, typename R>
-__device__ __forceinline__ Pair<R> ld_pair(const R* p, int i) {
-    if constexpr (VEC) {
-        static_assert(sizeof(R) == 8, "FP64 pairs");
-        const double2 v = *reinterpret_cast<const double2*>(p + i);
-        return {v.x, v.y};
-    } else {
-        return {p[i], p[i + 1]};
-    }
+template <bool VEC>
+__device__ __forceinline__ double2 ld_pair(const double* p, int i) {
+    if constexpr (VEC) return *reinterpret_cast<const double2*>(p + i);
+    return make_double2(p[i], p[i + 1]);
 }
-template <bool VEC, typename R>
-__device__ __forceinline__ void st_pair(R* p, int i, R a, R b, bool oka, bool okb) {
+template <bool VEC>
+__device__ __forceinline__ void st_pair(double* p, int i, double a, double b, bool oka, bool okb) {
     if (VEC && oka && okb) {
         *reinterpret_cast<double2*>(p + i) = make_double2(a, b);
     } else {
@@ -590,17 +581,17 @@ __host__ __device__ __forceinline__ unsigned xpair_blocks(const Box& b) {
 
 // cell c's weights; TVD slopes count on 0..n+1 only, and beyond it the weights
 // of the nearest such cell keep them on the rounded path
-template <int RECON, typename R>
-__device__ __forceinline__ CellWeights<RECON, R> xpair_weights(const AxisTabs& A, int c, int n) {
-    if constexpr (RECON == 4) return CellWeights<RECON, R>(A, c, c);
-    else return CellWeights<RECON, R>(A, min(max(c, 0), n + 1));
+template <int RECON>
+__device__ __forceinline__ CellWeights<RECON, double> xpair_weights(const AxisTabs& A, int c, int n) {
+    if constexpr (RECON == 4) return CellWeights<RECON, double>(A, c, c);
+    else return CellWeights<RECON, double>(A, min(max(c, 0), n + 1));
 }
 
-template <int RECON, typename R, bool RECIP, bool VEC>
-__global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box b, Tabs T, PrimT<R> pr, R ggas,
-                                                                           FaceFluxT<R> out, int l_lo, int l_step) {
+template <int RECON, bool RECIP, bool VEC>
+__global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box b, Tabs T, Prim pr, double ggas,
+                                                                           FaceFlux out, int l_lo, int l_step) {
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ R sm[28][XP_THREADS];  // states of the pair's two faces: left 7, right 7 each
+    __shared__ double sm[28][XP_THREADS];  // states of the pair's two faces: left 7, right 7 each
     const int cells = b.SX * (b.ny + 2);
     const unsigned bpp = xpair_blocks(b), plane = blockIdx.x / bpp;  // blocks a plane
     const int w = (int)(blockIdx.x - plane * bpp) * (XP_THREADS / 32) + (int)(threadIdx.x >> 5);
@@ -613,26 +604,26 @@ __global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box
     const bool ok0 = faces && m < cells && j0 >= 0 && j0 <= b.nx;
     const bool ok1 = faces && m + 1 < cells && j1 >= 0 && j1 <= b.nx;
     const AxisTabs A = T.ax[0];
-    const R* src[7] = {pr.w[0], pr.w[1], pr.w[2], pr.w[3], pr.w[4], pr.bc[1], pr.bc[2]};
-    const auto W0 = xpair_weights<RECON, R>(A, j0, b.nx), W1 = xpair_weights<RECON, R>(A, j1, b.nx);
+    const double* src[7] = {pr.w[0], pr.w[1], pr.w[2], pr.w[3], pr.w[4], pr.bc[1], pr.bc[2]};
+    const auto W0 = xpair_weights<RECON>(A, j0, b.nx), W1 = xpair_weights<RECON>(A, j1, b.nx);
 #pragma unroll
     for (int v = 0; v < 7; ++v) {
-        const Pair<R> x = ld_pair<VEC>(src[v], g);
-        const R xm = __shfl_up_sync(FULL, x.b, 1), xp = __shfl_down_sync(FULL, x.a, 1);
-        R vm0, vp0, vm1, vp1;
+        const double2 x = ld_pair<VEC>(src[v], g);
+        const double xm = __shfl_up_sync(FULL, x.y, 1), xp = __shfl_down_sync(FULL, x.x, 1);
+        double vm0, vp0, vm1, vp1;
         if constexpr (RECON == 4) {
-            const R d0 = W0.slope(xm, x.a, x.b), d1 = W1.slope(x.a, x.b, xp);
-            const R d2 = __shfl_down_sync(FULL, d0, 1);
-            const R V0 = W0.face(x.a, x.b, d0, d1), V1 = W1.face(x.b, xp, d1, d2);
-            const R Vm = __shfl_up_sync(FULL, V1, 1);
-            ppm_fix(x.a, Vm, V0, vm0, vp0);
-            ppm_fix(x.b, V0, V1, vm1, vp1);
+            const double d0 = W0.slope(xm, x.x, x.y), d1 = W1.slope(x.x, x.y, xp);
+            const double d2 = __shfl_down_sync(FULL, d0, 1);
+            const double V0 = W0.face(x.x, x.y, d0, d1), V1 = W1.face(x.y, xp, d1, d2);
+            const double Vm = __shfl_up_sync(FULL, V1, 1);
+            ppm_fix(x.x, Vm, V0, vm0, vp0);
+            ppm_fix(x.y, V0, V1, vm1, vp1);
         } else {
-            const R s0 = W0.slope(xm, x.a, x.b), s1 = W1.slope(x.a, x.b, xp);
-            vm0 = x.a - R(0.5) * s0;
-            vp0 = x.a + R(0.5) * s0;
-            vm1 = x.b - R(0.5) * s1;
-            vp1 = x.b + R(0.5) * s1;
+            const double s0 = W0.slope(xm, x.x, x.y), s1 = W1.slope(x.x, x.y, xp);
+            vm0 = x.x - 0.5 * s0;
+            vp0 = x.x + 0.5 * s0;
+            vm1 = x.y - 0.5 * s1;
+            vp1 = x.y + 0.5 * s1;
         }
         sm[v][tid] = vp0;  // face 2i | 2i+1: vp_out of its left cell, vm_out of its right cell
         sm[7 + v][tid] = vm1;
@@ -640,20 +631,20 @@ __global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box
         sm[21 + v][tid] = __shfl_down_sync(FULL, vm0, 1);
     }
     if (!ok0 && !ok1) return;
-    const Pair<R> bn = ld_pair<VEC>(pr.bf[0], g);
-    R fx[7];
+    const double2 bn = ld_pair<VEC>(pr.bf[0], g);
+    double fx[7];
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
         if (f == 0 ? ok0 : ok1) {
             constexpr int slot[7] = {IRHO, IVX, IVY, IVZ, ITAU, IBY, IBZ};
-            R wl[8], wr[8];
+            double wl[8], wr[8];
 #pragma unroll
             for (int v = 0; v < 7; ++v) {
                 wl[slot[v]] = sm[14 * f + v][tid];
                 wr[slot[v]] = sm[14 * f + 7 + v][tid];
             }
-            wl[IBX] = wr[IBX] = f == 0 ? bn.a : bn.b;
-            sweep_hll<0, R, RECIP>(wl, wr, ggas, fx);
+            wl[IBX] = wr[IBX] = f == 0 ? bn.x : bn.y;
+            sweep_hll<0, double, RECIP>(wl, wr, ggas, fx);
         }
         if (f == 0) {
 #pragma unroll
@@ -665,12 +656,11 @@ __global__ void __launch_bounds__(XP_THREADS, CUMC_XPAIR_MINB) k_sweep_xpair(Box
 }
 
 // the vector form's conditions: every pair aligned to its own size
-template <typename R>
-inline bool xpair_vec(const Box& b, const PrimT<R>& pr, const FaceFluxT<R>& out) {
+inline bool xpair_vec(const Box& b, const Prim& pr, const FaceFlux& out) {
     uintptr_t at = (uintptr_t)pr.bc[1] | (uintptr_t)pr.bc[2] | (uintptr_t)pr.bf[0];
     for (int q = 0; q < 5; ++q) at |= (uintptr_t)pr.w[q];
     for (int q = 0; q < 7; ++q) at |= (uintptr_t)out.f[q];
-    return b.SX % 2 == 0 && at % (2 * sizeof(R)) == 0;
+    return b.SX % 2 == 0 && at % 16 == 0;
 }
 inline dim3 xpair_grid(const Box& b, int l_cnt) { return dim3(xpair_blocks(b) * (unsigned)l_cnt); }
 
