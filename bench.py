@@ -126,14 +126,16 @@ def algorithmic_bytes(kernel: str, nx: int, ny: int, nz: int) -> float:
         return 8.0 * (7 * cells + faces + 7 * faces)
     box1 = (nx + 1) * (ny + 1) * (nz + 1)
     box2 = (nx + 2) * (ny + 2) * (nz + 2)
-    if kernel == "emf":
+    if kernel == "emf":  # k_emf, where the edge EMFs are a kernel of their own (CUMC_SWEEP variants)
         return 8.0 * (6 * box2 + 6 * box2 + 3 * box1)
-    if kernel == "combine":  # hydro combine + conversions, stage 2/3 form: 15 hydro fluxes, u0 and uc
-        # hydro, 3 face fields in; hydro cons, w, bcell, eps out. Stages 1 and 2 of a whole step leave
-        # out 4 hydro cons and eps: the mean over a step's three launches
-        return 8.0 * (15 + 5 + 5 + 3 + 5 + 5 + 3 + 1 - 2 * 5 / 3) * box1
-    if kernel == "ct":  # 3 EMF, u0 and uc face fields in, face fields out (stage 2/3 form)
-        return 8.0 * (3 + 3 + 3 + 3) * box1
+    if kernel == "combine":  # hydro combine + conversions, the mean over a step's three launches.
+        # In: 15 hydro fluxes, 5 u0, 3 face fields and, at stages 2 and 3, 5 for uc (the energy and
+        # the primitives that give the rest). Out: 5 w and 3 bcell; the energy at stages 1 and 2, 5
+        # hydro cons and eps at stage 3 (eps three cells deep before is left out)
+        return 8.0 * (15 + 5 + 3 + 2 * 5 / 3 + 5 + 3 + (1 + 1 + 6) / 3) * box1
+    if kernel == "ct":  # k_emf_ct (edge EMFs and CT), the mean over a step's three launches: 6 fluxes and
+        # 6 cell fields, u0 and, at stages 2 and 3, uc face fields in, face fields out
+        return 8.0 * (12 * box2 + (3 + 2 + 3) * box1)
     if kernel == "utop":
         return 8.0 * (8 + 2 + 5 + 5 + 1 + 3) * box1
     if kernel == "boundary":
