@@ -64,7 +64,11 @@ struct WalkGeom {
 // makes rounds x (faces + 1.5) least. Against about 64 faces, halved down to
 // 8 while the grid gave fewer than 32 warps a SM: 64^3 0.036 -> 0.029 ms a
 // walk, the 90x26x75 torus 0.029 -> 0.023, a 512x4x4 tube 0.021 -> 0.013; 256^3
-// unchanged (0.90).
+// unchanged (0.90). In a step's graph, where the three sweeps run side by side,
+// ms a step with that rule, this one, and this one with a third of the GPU a
+// sweep: 64^3 0.331, 0.328, 0.340; tube 0.125, 0.111, 0.111; 90x26x75 0.271,
+// 0.263, 0.266; 192x128x64 torus 1.720, 1.713, 1.702; 128^3 reciprocal solve
+// 1.760, 1.770, 1.781.
 constexpr int WK_RESIDENT = 10, WK_SEG_MAX = 64;  // (64 faces: 1.5 KB of FP32 weights a mixed block)
 template <int DIR>
 inline int walk_segment_for(const Box& b, long long ncols, int sm_count, int* nseg) {
