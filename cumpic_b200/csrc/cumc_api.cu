@@ -830,6 +830,7 @@ cudaError_t capture_rk_step(cumc_ctx* c) {
 constexpr int RK_GRAPH_CALL = 7;
 void rk_step_host(cumc_ctx* c, bool captured) {
     if (!c->prof_on && !captured && !c->rk_plain && (c->rk_exec || ++c->rk_calls >= RK_GRAPH_CALL)) {
+        const NvtxRange range("cumc rk step");
         if ((c->rk_exec || capture_rk_step(c) == cudaSuccess) &&
             cudaGraphLaunch(c->rk_exec, c->stream) == cudaSuccess) {
             c->launches += c->rk_launches;
