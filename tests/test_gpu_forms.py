@@ -75,6 +75,20 @@ extern "C" int cfl(long n, const double* w, double g, double number, const doubl
     return rc;
 }
 
+__global__ void k_recip(long n, const double* x, double* out) {
+    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (i < n) out[i] = recip_q<true>(x[i]);
+}
+extern "C" int recip(long n, const double* x, double* out) {
+    double* d;
+    if (cudaMalloc(&d, 2 * n * sizeof(double))) return 1;
+    cudaMemcpy(d, x, n * sizeof(double), cudaMemcpyHostToDevice);
+    k_recip<<<(unsigned)((n + 127) / 128), 128>>>(n, d, d + n);
+    const int rc = cudaMemcpy(out, d + n, n * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(d);
+    return rc;
+}
+
 // x: five cells, then two weights of a slope and (cf, cb) of a TVD cell
 __global__ void k_limit(long n, const double* x, double* out) {
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -254,6 +268,14 @@ def test_recip_solve_at_faint_fields_and_extreme_states(lib64):
     for d, (f, ref, scale) in enumerate(_hll(lib64.hll_recip, w, ctypes.c_double(GGAS), np.float64)):
         bad = ~(np.abs(f - ref) <= RECIP_TOL * scale + 1e-320).all(axis=1)
         assert not bad.any(), (d, bad.sum(), w[bad][0], f[bad][0], ref[bad][0], scale[bad][0])
+
+
+def test_reciprocals_are_rounded_to_nearest(lib64):
+    rng = np.random.default_rng(8)
+    x = (1.0 + rng.random(1_000_000)) * 2.0 ** rng.integers(-400, 400, 1_000_000)
+    out = np.empty_like(x)
+    assert lib64.recip(ctypes.c_long(len(x)), _p(x), _p(out)) == 0
+    assert np.array_equal(out, 1.0 / x)
 
 
 def test_recip_solve_keeps_non_finite_speeds(lib64):
