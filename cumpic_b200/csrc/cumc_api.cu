@@ -797,11 +797,18 @@ void rk_step_dt(cumc_ctx* c, const Box& b) {
 }
 
 // one rk_step_dt recorded into c->rk_exec; the context's stream keeps running as
-// before if that fails
+// before if that fails. (Instantiating allocates, which would invalidate a
+// capture that the caller has open on another stream: the thread's capture mode
+// is relaxed meanwhile.)
 cudaError_t capture_rk_step(cumc_ctx* c) {
     cudaGraph_t g = nullptr;
-    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return e;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed);
+    if (e != cudaSuccess) {
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        return e;
+    }
     const long long before = c->launches;
     c->fork = true;
     rk_step_dt(c, c->box);
@@ -812,6 +819,7 @@ cudaError_t capture_rk_step(cumc_ctx* c) {
     if (e == cudaSuccess) e = cudaGraphInstantiate(&c->rk_exec, g, 0);
     if (e != cudaSuccess) c->rk_exec = nullptr;
     if (g) cudaGraphDestroy(g);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     return e;
 }
 

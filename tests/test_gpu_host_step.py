@@ -142,3 +142,22 @@ def test_negative_radii():
         g.rungekutta(1e-4)
         o.rungekutta(1e-4)
     _same(g, o)
+
+
+def test_steps_beside_another_streams_capture():
+    """a capture that the caller has open on a stream of its own (global mode)
+    survives the step whose graph is made"""
+    import torch
+    g, o = _pair(P.orszag_tang(12, ny=9, nz=10))
+    x = torch.zeros(8, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        x += 1.0
+        for _ in range(9):
+            g.rungekutta(1e-3)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 1.0
+    for _ in range(9):
+        o.rungekutta(1e-3)
+    _same(g, o)
